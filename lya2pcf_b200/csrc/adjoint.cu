@@ -7,13 +7,12 @@
 // and symmetrically for j.  Bins with W_b == 0 contribute nothing (xi_b = 0,
 // as post_processing.py:147 defines it).
 //
-// Gather form: the work queue is walked in both directions, (f1, f2) and
-// (f2, f1); a warp owns the first forest of each item and sums the gradient of
-// its pixels in registers (one lane per pixel i, walking j), so no pixel pair
-// scatters into memory.  The pair bin is symmetric under the swap (|dc1-dc2|,
-// dc1+dc2 and the FMA-ordered cos12 are), so both directions see the same bin.
-// Bins are evaluated with the reference FP64 formula.  With sorted dc, the j
-// loop is limited to the window where rp < rpmax and rt < rtmax.
+// Two kernels share the work queue.  k_adjoint_band takes every pair of forests
+// whose dc are sorted, finite and not negative (the LYA_LEAN flag) and serves
+// both forests of a pair in one pass; k_adjoint takes the others: the gather
+// form, walked in both directions, one lane per pixel i over its partners j,
+// every bin from the reference FP64 formula.  The pair bin is symmetric under
+// the swap (|dc1-dc2|, dc1+dc2 and the FMA-ordered cos12 are).
 #include <algorithm>
 #include <cmath>
 
@@ -36,6 +35,7 @@ struct AdjParams {
   int64_t n_items;
   double binner_rp, binner_rt;
   int np, nt, nb, cos_variant;
+  int skip_lean;                     // k_adjoint: leave the pairs k_adjoint_band takes
   const double* __restrict__ coef;   // [2][nb]: g/W, -g xi/W
   double* __restrict__ g_dw;         // padded pixel layout
   double* __restrict__ g_w;
@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(256) k_adjoint(const AdjParams p) {
     const int64_t k = rev ? t - p.n_items : t;
     const int fa = rev ? p.f2[k] : p.f1[k];
     const int fb = rev ? p.f1[k] : p.f2[k];
+    if (p.skip_lean && (p.sorted[fa] & p.sorted[fb] & LYA_LEAN)) continue;
     const int L1 = p.len[fa], L2 = p.len[fb];
     if (L1 <= 0 || L2 <= 0) continue;
     const int64_t a = p.pstart[fa], b = p.pstart[fb];
@@ -162,6 +163,284 @@ __global__ void __launch_bounds__(256) k_adjoint(const AdjParams p) {
   }
 }
 
+// ------------------------------------------------------------------ pairs of lean forests
+// One warp per forest pair, 64 rows (f1 pixels) at a time: lane l holds rows
+// r = i0 + 2l and r + 1 and at step m the f2 pixel j = r + m, so all lanes are
+// on the same two diagonals, nearly the same |dc1 - dc2|, and cross the rp edges
+// within a step or two of one another.
+// * Bins: x = dc_j - dc_i and s = dc_j + dc_i grow with m, so each row walks the
+//   pair's rp edges (both signs of x) and rt edges upwards, comparing x and s
+//   with the next exact edge (lya_edge) instead of forming the bin of every
+//   pixel pair.  The steps of a row's rt edges, at most a few, are found before
+//   the walk, which leaves one FP64 addition and one comparison per pair.
+// * Gradients: a row's sums stay in its lane.  The sums of pixel j move one
+//   lane down every second step (two sets, even and odd steps), leave at lane 0
+//   into a ring of 32 pixels and go to memory 32 pixels at a time.
+// * f2 pixels pass through a ring in shared memory, even and odd pixels apart,
+//   so that the lanes' reads (two pixels apart) are conflict-free.
+// Bound: issue (69% of cycles) with shared-memory wavefronts at 55% and the FP64
+// pipe at 19% (6 operations per pixel pair for both directions; the gather form
+// needs 28).  One gradient of 2.80e10 pixel pairs (2,500 forests of 374 pixels):
+// 62.8 ms, the gather form over both directions 99.6 ms; 1.85e9 pairs of
+// 200-pixel forests: 6.0 against 8.6 ms.  24 warps at 80 registers: 20 warps
+// take 70 ms, 28 warps 64.5 ms, 32 warps 67.4 ms.
+constexpr int BAND_WARPS = 24;   // at most (80 registers)
+constexpr int BAND_RING = 128;   // f2 pixels in a warp's ring: 64 in use, 32 ahead, 32 spare
+
+// Shared memory, as offsets in doubles: the coefficients (2 values) of the nt
+// bins of every number of rp edges passed (0 .. 2 np, the first and the last out
+// of range), then per warp the ring (w, dw) of even and odd pixels, the ring's distances, the (grad dw, grad w) of 32 finished f2
+// pixels, the rp edges [2 np + 1] and the rt edges [nt + 1].
+constexpr int BAND_D = 2 * BAND_RING, BAND_OUT = BAND_D + BAND_RING, BAND_EX = BAND_OUT + 64;
+__host__ __device__ __forceinline__ int band_table(int np, int nt) { return 2 * (2 * np + 1) * nt; }
+__host__ __device__ __forceinline__ int band_per_warp(int np, int nt) { return BAND_EX + ((2 * np + 1 + nt + 1 + 1) & ~1); }
+extern __shared__ __align__(16) double s_band[];
+
+// Bin state of a row: the shared-memory offsets ox of the next rp edge and oc of
+// the bin's coefficients, the next rp edge, and the steps kt of its next four rt
+// edges (16 bits each, the nearest lowest).  The row's partners are in range on
+// steps kb .. kb + kn - 1.
+struct BandRow {
+  double d, w, dw;
+  double ex;
+  double gdw, gw;
+  unsigned long long kt;
+  int ox, oc, kb, kn;
+};
+
+__device__ __forceinline__ int edges_passed(int e, int n, double v) {   // entries of s_band[e .. e + n) that are <= v
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (v >= s_band[e + mid]) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+__device__ __forceinline__ void band_sums(BandRow& r, int k, const double2& wdw, double& jdw, double& jw) {
+  const double2 c = *reinterpret_cast<const double2*>(&s_band[r.oc]);
+  if ((unsigned)(k - r.kb) < (unsigned)r.kn) {
+    r.gdw = __fma_rn(c.x, wdw.y, r.gdw);
+    r.gw = __fma_rn(c.y, wdw.x, r.gw);
+    jdw = __fma_rn(c.x, r.dw, jdw);
+    jw = __fma_rn(c.y, r.w, jw);
+  }
+}
+
+// Pass the edges up to the pixel at distance d2, step k.  SINGLE: at most one rp
+// and one rt edge per step (half of the lanes pass an rp edge at each step of
+// 2 Mpc/h) and at most four rt edges per row, whose steps are known: no branch.
+template <bool SINGLE>
+__device__ __forceinline__ void band_edges(BandRow& r, double d2, int k, int nt2, int es) {
+  const double x = __dsub_rn(d2, r.d);
+  if (SINGLE) {
+    if (x >= r.ex) { ++r.ox; r.oc += nt2; }
+    r.ex = s_band[r.ox];
+    if (k == (int)(r.kt & 0xffff)) { r.oc += 2; r.kt >>= 16; }
+  } else {
+    while (x >= r.ex) { r.ex = s_band[++r.ox]; r.oc += nt2; }
+    const double s = __dadd_rn(d2, r.d);
+    while (s >= s_band[es + (int)r.kt]) { ++r.kt; r.oc += 2; }   // kt: rt edges passed
+  }
+}
+
+// The pixel pairs of both rows and the f2 pixel at ring position q of parity
+// par (step k), whose sums are jdw, jw.
+template <bool SINGLE>
+__device__ __forceinline__ void band_pair(BandRow& ra, BandRow& rb, int ring, int par, int q, int k, double& jdw,
+                                          double& jw, int nt2, int es) {
+  const double2 wdw = *reinterpret_cast<const double2*>(&s_band[ring + par * BAND_RING + 2 * q]);
+  const double d2 = s_band[ring + BAND_D + par * (BAND_RING / 2) + q];
+  band_edges<SINGLE>(ra, d2, k, nt2, es);
+  band_edges<SINGLE>(rb, d2, k, nt2, es);
+  band_sums(ra, k, wdw, jdw, jw);
+  band_sums(rb, k, wdw, jdw, jw);
+}
+
+// Sums of the f2 pixels of the current two steps (even, odd), one pixel per lane each.
+struct BandCols {
+  double pdw, pw, qdw, qw;
+};
+
+// n steps (rounded up to even: a step past the band meets only pairs out of
+// range or outside the forest) from ring position k0.
+template <bool SINGLE>
+__device__ __forceinline__ void band_walk(BandRow& ra, BandRow& rb, BandCols& c, int ring, int k0, int n, int nt2, int es) {
+  const int lane = threadIdx.x & 31;
+  for (int k = 0; k < n; k += 2) {
+    const int q = (((k0 + k) >> 1) + lane) & (BAND_RING / 2 - 1);
+    band_pair<SINGLE>(ra, rb, ring, 0, q, k0 + k, c.pdw, c.pw, nt2, es);
+    band_pair<SINGLE>(ra, rb, ring, 1, q, k0 + k + 1, c.qdw, c.qw, nt2, es);
+    if (lane == 0) {
+      *reinterpret_cast<double2*>(&s_band[ring + BAND_OUT + 2 * k]) = make_double2(c.pdw, c.pw);
+      *reinterpret_cast<double2*>(&s_band[ring + BAND_OUT + 2 * k + 2]) = make_double2(c.qdw, c.qw);
+    }
+    c.pdw = __shfl_down_sync(0xffffffffu, c.pdw, 1); c.pw = __shfl_down_sync(0xffffffffu, c.pw, 1);
+    c.qdw = __shfl_down_sync(0xffffffffu, c.qdw, 1); c.qw = __shfl_down_sync(0xffffffffu, c.qw, 1);
+    if (lane == 31) { c.pdw = 0.0; c.pw = 0.0; c.qdw = 0.0; c.qw = 0.0; }
+  }
+}
+
+__global__ void __launch_bounds__(BAND_WARPS * 32, 1) k_adjoint_band(const AdjParams p) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int np = p.np, nt = p.nt, nb = p.nb;
+  for (int k = threadIdx.x; k < (2 * np + 1) * nt; k += blockDim.x) {
+    const int q = abs(k / nt - np) * nt + k % nt;
+    s_band[2 * k] = q < nb ? p.coef[q] : 0.0;
+    s_band[2 * k + 1] = q < nb ? p.coef[nb + q] : 0.0;
+  }
+  const int nt2 = 2 * nt;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ring = band_table(np, nt) + warp * band_per_warp(np, nt);
+  const int ex = ring + BAND_EX, es = ex + 2 * np + 1;
+  const double NaN = __longlong_as_double(0x7ff8000000000000ll), INF = __longlong_as_double(0x7ff0000000000000ll);
+  __syncthreads();
+  const int warps = blockDim.x >> 5;
+  const int64_t nw = (int64_t)gridDim.x * warps;
+  for (int64_t t = blockIdx.x * (int64_t)warps + warp; t < p.n_items; t += nw) {
+    const int fa = p.f1[t], fb = p.f2[t];
+    if (!(p.sorted[fa] & p.sorted[fb] & LYA_LEAN)) continue;
+    const int L1 = p.len[fa], L2 = p.len[fb];
+    if (L1 <= 0 || L2 <= 0) continue;
+    const int64_t a = p.pstart[fa], b = p.pstart[fb];
+    double c = lya_cos12(p.ux[fa], p.uy[fa], p.uz[fa], p.ux[fb], p.uy[fb], p.uz[fb], p.cos_variant);
+    c = fmin(1.0, fmax(-1.0, c));
+    const double ch = __dsqrt_rn(__dmul_rn(0.5, __dadd_rn(1.0, c)));
+    const double sh = __dsqrt_rn(__dmul_rn(0.5, __dsub_rn(1.0, c)));
+    __syncwarp();   // every lane is done with the previous pair's edges
+    // passing edge k: x < 0 enters rp bin np - 1 - k (k < np), x >= 0 bin k - np + 1
+    for (int k = lane; k < np; k += 32) {
+      const double e = lya_edge((double)(k + 1), ch, p.binner_rp);   // |x| >= e: bin k + 1 or above
+      s_band[ex + np - 1 - k] = -lya_below(e);
+      s_band[ex + np + k] = e;
+    }
+    for (int k = lane; k < nt; k += 32) s_band[es + k] = lya_edge((double)(k + 1), sh, p.binner_rt);
+    if (lane == 0) { s_band[ex + 2 * np] = INF; s_band[es + nt] = INF; }
+    __syncwarp();
+    // in range: x_lo <= x < x_hi, s < s_hi
+    const double x_lo = s_band[ex], x_hi = s_band[ex + 2 * np - 1], s_hi = s_band[es + nt - 1];
+    const double* __restrict__ D2 = p.dc + b;
+    const double* __restrict__ W2 = p.w + b;
+    const double* __restrict__ DW2 = p.dw + b;
+    double gap = 0.0;   // largest step along f2
+    for (int k = lane; k + 1 < L2; k += 32) gap = fmax(gap, D2[k + 1] - D2[k]);
+    const bool one_edge = __all_sync(FULL, gap * ch * p.binner_rp < 0.999 && gap * sh * p.binner_rt < 0.999);
+    for (int i0 = 0; i0 < L1; i0 += 64) {
+      BandRow ra, rb;
+      const int i = i0 + 2 * lane;
+      // the rows' diagonals: first and last partner in range (x and s grow with j)
+      int m_lo = INT_MAX, m_hi = INT_MIN, first_ss = 0, second_ss = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        BandRow& r = h ? rb : ra;
+        const bool ok = i + h < L1;
+        r.d = ok ? p.dc[a + i + h] : NaN;
+        r.w = ok ? p.w[a + i + h] : 0.0;
+        r.dw = ok ? p.dw[a + i + h] : 0.0;
+        r.gdw = 0.0; r.gw = 0.0;
+        if (ok) {
+          int lo = 0, hi = L2;
+          while (lo < hi) { const int k = (lo + hi) >> 1; if (__dsub_rn(D2[k], r.d) >= x_lo) hi = k; else lo = k + 1; }
+          const int j0 = lo;
+          hi = L2;
+          while (lo < hi) {
+            const int k = (lo + hi) >> 1;
+            if (__dsub_rn(D2[k], r.d) >= x_hi || __dadd_rn(D2[k], r.d) >= s_hi) hi = k; else lo = k + 1;
+          }
+          if (lo > j0) {
+            m_lo = min(m_lo, j0 - i);      // step m of row h has partner i + m
+            m_hi = max(m_hi, lo - 1 - i);
+          }
+          r.kb = j0;                       // as pixels of f2 until m_lo is known
+          r.kn = lo - j0;
+        } else {
+          r.kb = 0;
+          r.kn = 0;
+        }
+      }
+      m_lo = __reduce_min_sync(FULL, m_lo);
+      m_hi = __reduce_max_sync(FULL, m_hi);
+      if (m_lo > m_hi) continue;
+      // bin states before the first step: as of the first partner there is
+      const int steps = m_hi - m_lo + 1;
+      bool single = one_edge && steps < 0xffff;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        BandRow& r = h ? rb : ra;
+        const int j = max(0, i + m_lo);
+        const double d2 = j < L2 ? D2[j] : NaN;
+        const int sx = edges_passed(ex, 2 * np, __dsub_rn(d2, r.d));
+        // the rt bin as of the first partner in range
+        const int ss = r.kn > 0 ? edges_passed(es, nt, __dadd_rn(D2[r.kb], r.d)) : 0;
+        r.ox = ex + sx;
+        r.oc = sx * nt2 + 2 * ss;
+        r.ex = s_band[r.ox];
+        r.kt = ~0ull;
+        int at = r.kb;   // the row's partners are at, at + 1, ... end - 1
+        const int end = r.kb + r.kn;
+        for (int q = 0; at < end; ++q) {   // steps of the rt edges the row passes
+          const double e = s_band[es + ss + q];
+          int hi = end;
+          while (at < hi) { const int k = (at + hi) >> 1; if (__dadd_rn(D2[k], r.d) >= e) hi = k; else at = k + 1; }
+          if (at == end) break;
+          if (q == 4) { single = false; break; }
+          r.kt = (r.kt & ~(0xffffull << 16 * q)) | (unsigned long long)(at - i - m_lo) << 16 * q;
+        }
+        if (h) second_ss = ss; else first_ss = ss;
+        r.kb -= i + m_lo;
+      }
+      single = __all_sync(FULL, single);
+      if (!single) { ra.kt = first_ss; rb.kt = second_ss; }
+      // pixels jb .. jb + 31 of f2 into the ring (pixels outside the forest: NaN, no weight)
+      const int j00 = i0 + m_lo;      // lane 0's partner at step 0
+      auto stage = [&](int k0) {
+        const int j = j00 + k0 + lane, q = (k0 + lane) & (BAND_RING - 1);
+        const bool ok = j >= 0 && j < L2;
+        s_band[ring + BAND_D + (q & 1) * (BAND_RING / 2) + (q >> 1)] = ok ? D2[j] : NaN;
+        *reinterpret_cast<double2*>(&s_band[ring + (q & 1) * BAND_RING + 2 * (q >> 1)]) =
+            ok ? make_double2(W2[j], DW2[j]) : make_double2(0.0, 0.0);
+      };
+      __syncwarp();
+      stage(0);
+      stage(32);
+      BandCols col = {0.0, 0.0, 0.0, 0.0};
+      for (int k0 = 0; k0 < steps; k0 += 32) {
+        stage(k0 + 64);
+        __syncwarp();
+        const int n = min(32, steps - k0);
+        if (single) band_walk<true>(ra, rb, col, ring, k0, n, nt2, es);
+        else band_walk<false>(ra, rb, col, ring, k0, n, nt2, es);
+        __syncwarp();
+        const int j = j00 + k0 + lane;
+        if (lane < ((n + 1) & ~1) && j >= 0 && j < L2) {
+          const double2 g = *reinterpret_cast<const double2*>(&s_band[ring + BAND_OUT + 2 * lane]);
+          if (g.x != 0.0) atomicAdd(&p.g_dw[b + j], g.x);
+          if (g.y != 0.0) atomicAdd(&p.g_w[b + j], g.y);
+        }
+        __syncwarp();
+      }
+      // the f2 pixels still in the lanes, and the rows
+      const int js = j00 + ((steps + 1) & ~1) + 2 * lane;
+      if (js >= 0 && js < L2) {
+        if (col.pdw != 0.0) atomicAdd(&p.g_dw[b + js], col.pdw);
+        if (col.pw != 0.0) atomicAdd(&p.g_w[b + js], col.pw);
+      }
+      if (js + 1 >= 0 && js + 1 < L2) {
+        if (col.qdw != 0.0) atomicAdd(&p.g_dw[b + js + 1], col.qdw);
+        if (col.qw != 0.0) atomicAdd(&p.g_w[b + js + 1], col.qw);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const BandRow& r = h ? rb : ra;
+        if (i + h < L1) {
+          if (r.gdw != 0.0) atomicAdd(&p.g_dw[a + i + h], r.gdw);
+          if (r.gw != 0.0) atomicAdd(&p.g_w[a + i + h], r.gw);
+        }
+      }
+    }
+  }
+}
+
 __global__ void k_unpad(int64_t n, const int64_t* __restrict__ start, const int64_t* __restrict__ pstart,
                         const double* __restrict__ src, double* __restrict__ dst) {
   for (int64_t f = blockIdx.x; f < n; f += gridDim.x) {
@@ -219,11 +498,29 @@ int lya_adjoint_launch(lya_ctx* ctx, const double* g, double* grad_dw, double* g
     p.binner_rp = (double)ctx->np / ctx->rpmax; p.binner_rt = (double)ctx->nt / ctx->rtmax;
     p.np = ctx->np; p.nt = ctx->nt; p.nb = nb; p.cos_variant = ctx->cos_variant;
     p.coef = coef; p.g_dw = gdw; p.g_w = gw;
-    const size_t smem = sizeof(double) * 2 * nb;
-    e = cudaFuncSetAttribute(k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && p.n_items > 0) {
-      k_adjoint<<<ctx->num_sms * 4, 256, smem, s>>>(p);
-      ctx->launches++;
+    // The band kernel takes the lean pairs when its table leaves shared memory
+    // for 8 warps or more (50 x 50 bins: 81 KB, 24 warps of 4.8 KB); the gather
+    // kernel takes the pairs it leaves.
+    const size_t smem = sizeof(double) * 2 * nb, smem_max = 226 * 1024;
+    const size_t table = sizeof(double) * (size_t)band_table(ctx->np, ctx->nt);
+    const size_t per_warp = sizeof(double) * (size_t)band_per_warp(ctx->np, ctx->nt);
+    const int warps = table < smem_max ? (int)std::min<size_t>(BAND_WARPS, (smem_max - table) / per_warp) : 0;
+    const bool band = warps >= 8;
+    p.skip_lean = band ? 1 : 0;
+    if (band && p.n_items > 0) {
+      const size_t smem_band = table + warps * per_warp;
+      e = cudaFuncSetAttribute(k_adjoint_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_band);
+      if (e == cudaSuccess) {
+        k_adjoint_band<<<ctx->num_sms, warps * 32, smem_band, s>>>(p);
+        ctx->launches++;
+      }
+    }
+    if (p.n_items > 0 && (!band || ctx->cat.n_not_lean > 0)) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) {
+        k_adjoint<<<ctx->num_sms * 4, 256, smem, s>>>(p);
+        ctx->launches++;
+      }
     }
     if (e == cudaSuccess) e = cudaGetLastError();
   }

@@ -261,6 +261,24 @@ __device__ __forceinline__ double lya_cos12(double x1, double y1, double z1, dou
   return __dadd_rn(__dadd_rn(__dmul_rn(x1, x2), __dmul_rn(y1, y2)), __dmul_rn(z1, z2));
 }
 
+// Exact bin edge of the reference formula: the smallest t >= 0 with
+// (t * c) * binner >= b in FP64 (each product rounded), +inf when no finite t
+// has it.  Both roundings are monotone, so t >= lya_edge(b) is the same test as
+// floor((t * c) * binner) >= b, and a comparison replaces the two products and
+// the floor of every pixel pair.  The quotient is within a few ulps of the
+// edge; the two loops step to it.
+__device__ __forceinline__ double lya_edge(double b, double c, double binner) {
+  double t = b / (c * binner);
+  if (!(t < 1.0e300)) return __longlong_as_double(0x7ff0000000000000ll);
+  long long u = __double_as_longlong(t);
+  while (u > 0 && __dmul_rn(__dmul_rn(__longlong_as_double(u - 1), c), binner) >= b) --u;
+  while (__dmul_rn(__dmul_rn(__longlong_as_double(u), c), binner) < b) ++u;
+  return __longlong_as_double(u);
+}
+
+// The double just below a positive t (below +inf: the largest finite one).
+__device__ __forceinline__ double lya_below(double t) { return __longlong_as_double(__double_as_longlong(t) - 1); }
+
 // D(8x8) += A(8x4) B(4x8) in FP64 on the tensor cores, one warp (FP64 has no
 // tcgen05 kind).  Fragments: a = A[lane/4][lane%4], b = B[lane%4][lane/4],
 // d = D[lane/4][2*(lane%4) + {0,1}].

@@ -1,0 +1,75 @@
+"""Kernels that walk the exact bin edges of sorted forests, against the oracle's
+per-pair reference formula, where a walk can go wrong: forest lengths around
+the 32- and 64-pixel chunks, pixels exactly on rp edges, pixel steps below and
+above a bin, bins so narrow in rt that a row meets many edges, one bin only,
+binnings that leave the walk to the general kernel, and forests that do."""
+import numpy as np
+import pytest
+
+from helpers import forestset
+from lya2pcf_b200 import _native as N
+from lya2pcf_b200.engine import PairEngine
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = (1, 2, 31, 32, 33, 63, 64, 65, 96, 127, 128, 129, 200, 330, 614)
+
+
+def ragged(step, unsorted=False, seed=5):
+    """Forests of LENGTHS pixels within half a degree, some coincident lines of
+    sight; distances on a common grid (so that differences fall exactly on rp
+    edges for coincident lines of sight) and a jittered copy of it."""
+    rng = np.random.default_rng(seed)
+    grid = 3600.0 + step * np.arange(1200) - 1e-4 * step * np.arange(1200) ** 2 / 8
+    exact = 3600.0 + step * np.arange(1200)
+    forests = []
+    for k, L in enumerate(LENGTHS):
+        o = int(rng.integers(0, 500))
+        dc = (exact if k % 3 == 0 else grid)[o:o + L].copy()
+        if k % 3 == 1:
+            dc += rng.uniform(0, 0.4 * step)
+        if unsorted and k % 4 == 2 and L > 2:
+            dc = dc[::-1].copy()
+        ra, dec = (0.5, 0.1) if k % 5 == 0 else (0.5 + rng.uniform(0, 0.03), 0.1 + rng.uniform(-0.02, 0.02))
+        forests.append(dict(ra=ra + 1e-9 * k, dec=dec, dc=dc, w=rng.uniform(0.5, 2.0, L), dw=rng.normal(0, 0.3, L),
+                            z=2.0 + 1e-3 * np.arange(L)))
+    return forestset(forests, pix=np.arange(len(LENGTHS)) // 6)
+
+
+def all_pairs(fs):
+    f1, f2 = np.triu_indices(fs.n, 1)
+    return f1.astype(np.int32), f2.astype(np.int32)
+
+
+BINNINGS = [
+    (50, 50, 2.0, False),      # steps of half an rp bin
+    (50, 50, 2.0, True),       # some forests unsorted: the general kernel for their pairs
+    (50, 50, 9.0, False),      # steps above a bin
+    (200, 16, 2.0, False),     # the same from narrow rp bins
+    (16, 200, 2.0, False),     # a row meets many rt edges
+    (1, 1, 2.0, False),
+    (64, 64, 2.0, False),      # largest binning of 64 rp bins
+    (4096, 1, 0.5, False),     # too many rp edges for shared memory
+]
+
+
+@pytest.mark.parametrize('np_,nt,step,unsorted', BINNINGS)
+def test_adjoint_edges(np_, nt, step, unsorted):
+    """Gradient against the oracle.  Both add the same products (<= 15 x 614
+    per pixel) in FP64 in different orders: 1e4 x 2^-53 of the largest
+    component's terms, 1e-11 of the largest component allowed."""
+    fs = ragged(step, unsorted)
+    f1, f2 = all_pairs(fs)
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        eng.run(kernel=N.KERNEL_FP64_PLAIN)
+        W, DW = eng.totals()
+        g = np.random.default_rng(7).normal(size=eng.nb)
+        gdw, gw = eng.adjoint(g)
+    cdw = np.divide(g, W, out=np.zeros_like(W), where=W != 0)
+    odw, ow = O.adjoint(fs, f1, f2, cdw, -cdw * np.divide(DW, W, out=np.zeros_like(W), where=W != 0), np_=np_, nt=nt)
+    assert np.abs(odw).max() > 0
+    np.testing.assert_allclose(gdw, odw, rtol=0, atol=1e-11 * np.abs(odw).max())
+    np.testing.assert_allclose(gw, ow, rtol=0, atol=1e-11 * np.abs(ow).max())
