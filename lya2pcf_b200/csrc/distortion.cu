@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NS = col_stride(np);
-  // q / (NS/2) as a multiply-high: exact for q < 2^16 (the copies of a chunk)
+  // q / (NS/2) as a multiply-high: exact for q < 2^16 (the copies of a chunk) and NS > 2
   const unsigned seg_magic = (unsigned)((0x100000000ull + (unsigned)(NS / 2) - 1) / (unsigned)(NS / 2));
   double* colS = p.col + (size_t)blockIdx.x * 2 * 2 * ML * TS * NS;   // [2 sides][ML][TS][NS]
   double* colL = colS + (size_t)2 * ML * TS * NS;
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           const int segs = NS / 2;                 // 16-byte segments of a row
           // q = (set CH + r) segs + sg over whole chunks; rows r >= rows are skipped
           for (int q = tid; q < nset * CH * segs; q += DT) {
-            const int sr = (int)__umulhi((unsigned)q, seg_magic), sg = q - sr * segs;
+            const int sr = segs > 1 ? (int)__umulhi((unsigned)q, seg_magic) : q, sg = q - sr * segs;
             const int set = sr / CH, r = sr - set * CH;
             if (r >= rows) continue;
             const double* colb = (set & 1) ? colL : colS;

@@ -73,3 +73,20 @@ def test_adjoint_edges(np_, nt, step, unsorted):
     assert np.abs(odw).max() > 0
     np.testing.assert_allclose(gdw, odw, rtol=0, atol=1e-11 * np.abs(odw).max())
     np.testing.assert_allclose(gw, ow, rtol=0, atol=1e-11 * np.abs(ow).max())
+
+
+@pytest.mark.parametrize('np_,nt,step,unsorted', [(50, 50, 2.0, False), (50, 50, 2.0, True), (50, 50, 9.0, False),
+                                                  (64, 16, 2.0, False), (33, 20, 2.0, False), (31, 20, 2.0, False),
+                                                  (1, 1, 2.0, False)])
+def test_distortion_edges(np_, nt, step, unsorted):
+    """D and W against the oracle's eta products: the tolerance of the other
+    distortion tests (1e-10 of max|D|, W to 1e-12)."""
+    fs = ragged(step, unsorted)
+    f1, f2 = all_pairs(fs)
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        D, W = eng.distortion()
+    Do, Wo = O.distortion(fs, f1, f2, np_=np_, nt=nt)
+    np.testing.assert_allclose(W, Wo, rtol=1e-12, atol=1e-12 * np.abs(Wo).max())
+    assert np.abs(D - Do).max() <= 1e-10 * np.abs(Do).max() and np.abs(Do).max() > 0
