@@ -62,7 +62,7 @@ def cov(xi, weight, device=0, numpix=None):
     n, nb = xi.shape
     np_, nt = _shape(nb, numpix)
     mean = np.zeros(nb)
-    c = np.zeros((nb, nb))
+    c = np.empty((nb, nb))   # filled by the library, which backs its pages beside the kernels
     with _Ctx(device, np_, nt) as k:
         rc = k.lib.lya_covariance(k.ctx, n, N.ptr(xi), N.ptr(weight), N.ptr(mean), N.ptr(c))
         if rc == 5:   # LYA_ERR_DATA: a bin with zero total weight
@@ -79,7 +79,7 @@ def cov_smooth(xi, weight, r_p, r_t, covariance_matrix, device=0, numpix=None):
     rp0, rt0 = bin_coordinates(np_, nt)
     if not (np.array_equal(np.asarray(r_p), rp0) and np.array_equal(np.asarray(r_t), rt0)):
         raise ValueError('r_p, r_t must be bin_coordinates(numpix_rp, numpix_rt)')
-    out = np.zeros_like(c)
+    out = np.empty_like(c)
     sm = C.c_int32(0)
     with _Ctx(device, np_, nt) as k:
         N.check(k.lib.lya_covariance_smooth(k.ctx, N.ptr(c), N.ptr(out), C.byref(sm)), k.ctx)

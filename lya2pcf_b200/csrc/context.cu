@@ -13,6 +13,8 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <thread>
 
 #include "lya_internal.cuh"
 
@@ -56,6 +58,29 @@ int lya_fail(lya_ctx* ctx, int code, const char* fmt, ...) {
   g_thread_err = buf;
   if (ctx) ctx->err = buf;
   return code;
+}
+
+void lya_touch_pages(void* p, size_t bytes) {
+  constexpr size_t PAGE = 4096, SHARE = size_t(1) << 20;
+  if (!p || bytes < 2 * SHARE) return;
+  auto touch = [p, bytes](size_t from, size_t to) {
+    for (size_t k = from; k < to && k < bytes; k += PAGE) __atomic_fetch_or(static_cast<char*>(p) + k, 0, __ATOMIC_RELAXED);
+  };
+  constexpr unsigned MOST = 8;
+  std::thread helpers[MOST - 1];
+  const unsigned n = std::min({MOST, std::max(1u, std::thread::hardware_concurrency() / 2), (unsigned)(bytes / SHARE)});
+  const size_t share = (bytes / n + PAGE) & ~(PAGE - 1);
+  unsigned started = 0;
+  try {
+    while (started + 1 < n) {
+      helpers[started] = std::thread(touch, (started + 1) * share, (started + 2) * share);
+      ++started;
+    }
+  } catch (const std::exception&) {   // no more threads: the rest is this one's
+  }
+  touch(0, share);
+  if (started + 1 < n) touch((started + 1) * share, bytes);
+  for (unsigned k = 0; k < started; ++k) helpers[k].join();
 }
 
 void lya_free_catalog(DevCatalog& c) {
@@ -172,10 +197,7 @@ extern "C" int lya_ctx_create(int device, lya_ctx** out) {
     if ((e = cudaEventCreate(&ctx->ev3)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
     if ((e = cudaEventCreate(&ctx->tev0)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
     if ((e = cudaEventCreate(&ctx->tev1)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
-    if ((e = lya_alloc(&ctx->stats, ST_N)) != cudaSuccess) { rc = LYA_ERR_ALLOC; break; }
-    if ((e = cudaMallocHost((void**)&ctx->h_stats, sizeof(unsigned long long) * (ST_N + 1))) != cudaSuccess) {
-      rc = LYA_ERR_ALLOC; break;
-    }
+    if ((e = lya_alloc(&ctx->stats, ST_N + 1)) != cudaSuccess) { rc = LYA_ERR_ALLOC; break; }
   } while (0);
   if (rc != LYA_OK) {
     lya_fail(nullptr, rc, "lya_ctx_create: %s", cudaGetErrorString(e));
@@ -204,11 +226,11 @@ extern "C" int lya_ctx_destroy(lya_ctx* ctx) {
   lya_free(ctx->hist); lya_free(ctx->counts); lya_free(ctx->stats); lya_free(ctx->cta_begin);
   lya_free(ctx->cost);
   lya_free(ctx->cov);
+  lya_free(ctx->covs.rows); lya_free(ctx->covs.bins); lya_free(ctx->covs.mat); lya_free(ctx->covs.zero);
   lya_free(ctx->dist.D); lya_free(ctx->dist.W); lya_free(ctx->dist.col); lya_free(ctx->dist.mom);
   lya_free(ctx->dist.err);
   if (ctx->dist.graph) cudaGraphExecDestroy(ctx->dist.graph);
   if (ctx->scan_tmp) cudaFree(ctx->scan_tmp);
-  if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
   if (ctx->run_graph) cudaGraphExecDestroy(ctx->run_graph);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -636,12 +658,14 @@ extern "C" int lya_corr_get(lya_ctx* ctx, int32_t slot_first, int32_t n, double*
     k_combine<<<blocks, 256, 0, ctx->stream>>>(n, nb, src, tmp);
     ctx->launches++;
     e = cudaGetLastError();
+    lya_touch_pages(hist, sizeof(double) * (size_t)n * LYA_NQ * nb);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(hist, tmp, sizeof(double) * (size_t)n * LYA_NQ * nb, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_corr_get: %s", cudaGetErrorString(e));
   }
   if (counts) {
+    lya_touch_pages(counts, sizeof(unsigned long long) * (size_t)n * nb);
     LYA_CHECK_CUDA(ctx, cudaMemcpyAsync(counts, ctx->counts + (size_t)slot_first * nb,
                                         sizeof(unsigned long long) * (size_t)n * nb, cudaMemcpyDeviceToHost,
                                         ctx->stream));

@@ -1256,9 +1256,8 @@ struct RunGraphKey {
 };
 
 // The stream work of one run: clear the outputs, balance the work queue over
-// the CTAs (cost prefix sum), the persistent pair kernel, and the copy of the
-// counters to pinned host memory.  No allocation and no synchronisation, so it
-// is captured once in a CUDA graph and replayed.
+// the CTAs (cost prefix sum), the persistent pair kernel.  No allocation and no
+// synchronisation, so it is captured once in a CUDA graph and replayed.
 static cudaError_t enqueue_run(lya_ctx* ctx, const RunGraphKey& k, double* d_range_pairs, int slot_begin,
                                int slot_end) {
   cudaStream_t s = ctx->stream;
@@ -1296,10 +1295,6 @@ static cudaError_t enqueue_run(lya_ctx* ctx, const RunGraphKey& k, double* d_ran
   }
   if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev1, s, cudaEventRecordExternal);
   if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev3, s, cudaEventRecordExternal);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->h_stats, p.stats, sizeof(unsigned long long) * ST_N, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->h_stats + ST_N, d_range_pairs, sizeof(double), cudaMemcpyDeviceToHost, s);
   return e;
 }
 
@@ -1338,8 +1333,7 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
       return lya_fail(ctx, LYA_ERR_ALLOC, "lya_corr_run: allocation failed");
     ctx->cta_cap = nctas + 2;
   }
-  // the range's reference pair count shares the cta_begin buffer
-  double* d_range_pairs = reinterpret_cast<double*>(ctx->cta_begin + nctas + 1);
+  double* d_range_pairs = reinterpret_cast<double*>(ctx->stats + ST_N);
   const int64_t n = ctx->wq.n_pairs;
   if (ctx->cost_cap < std::max<int64_t>(n, 1)) {
     lya_free(ctx->cost);
@@ -1424,6 +1418,8 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
   LYA_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->run_graph, s));
   // k_item_cost (when there are items), k_cta_bounds, the pair kernel (two instances with the rest pass)
   ctx->launches += (n > 0 ? 3 : 2) + key.rest_pass;
+  // the counters: one small copy to ordinary memory (pinned memory would cost every context 3 ms)
+  LYA_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_stats, ctx->stats, sizeof(ctx->h_stats), cudaMemcpyDeviceToHost, s));
   LYA_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
   float ms = 0.f, ms_all = 0.f;
   LYA_CHECK_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

@@ -147,12 +147,15 @@ __global__ void k_cov_steps(int nb, int np, int nt, const double* __restrict__ c
   }
 }
 
-__global__ void k_cov_smooth(int nb, int nt, const double* __restrict__ cov, const double* __restrict__ ssum,
-                             const double* __restrict__ scnt, double* __restrict__ out) {
+__global__ void k_cov_smooth(int nb, int nt, const double* cov, const double* __restrict__ ssum,
+                             const double* __restrict__ scnt, double* out) {   // out may be cov
   const int64_t total = (int64_t)nb * nb;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
     const int a = (int)(k / nb), b = (int)(k - (int64_t)a * nb);
-    if (a == b) { out[k] = cov[k]; continue; }
+    if (a == b) {
+      if (out != cov) out[k] = cov[k];
+      continue;
+    }
     const int pa = a / nt, qa = a - pa * nt, pb = b / nt, qb = b - pb * nt;
     const int st = abs(pb - pa) * nt + abs(qb - qa);
     const double norm = sqrt(cov[(size_t)a * nb + a] * cov[(size_t)b * nb + b]);
@@ -163,6 +166,23 @@ __global__ void k_cov_smooth(int nb, int nt, const double* __restrict__ cov, con
 __global__ void k_count_zero_diag(int nb, const double* __restrict__ cov, unsigned long long* __restrict__ zero) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
     if (cov[(size_t)b * nb + b] == 0.0) atomicAdd(zero, 1ull);
+}
+
+// Room for `rows` doubles of row data, nb bins and `mat` matrix entries.
+cudaError_t cov_reserve(CovScratch& c, int64_t rows, int nb, int64_t mat) {
+  cudaError_t e = cudaSuccess;
+  if (!c.zero) e = lya_alloc(&c.zero, 1);
+  auto grow = [&](double*& p, auto& cap, int64_t want, int64_t count) {
+    if (e != cudaSuccess || cap >= want) return;
+    lya_free(p);
+    cap = 0;
+    e = lya_alloc(&p, (size_t)count);
+    if (e == cudaSuccess) cap = want;
+  };
+  grow(c.rows, c.cap_rows, rows, rows);
+  grow(c.bins, c.cap_bins, nb, 2 * (int64_t)nb);
+  grow(c.mat, c.cap_mat, mat, mat);
+  return e;
 }
 
 }  // namespace
@@ -188,19 +208,11 @@ extern "C" int lya_covariance(lya_ctx* ctx, int64_t n_rows, const double* xi, co
     ctx->cov_nb = nb;
   }
   ctx->have_cov = false;
-  double *d_xi = nullptr, *d_w = nullptr, *d_y = nullptr, *d_W = nullptr, *d_mean = nullptr;
-  unsigned long long* d_zero = nullptr;
-  cudaError_t e = lya_alloc(&d_xi, (size_t)n * nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_w, (size_t)n * nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_y, (size_t)n * nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_W, nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_mean, nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_zero, 1);
-  auto cleanup = [&]() { lya_free(d_xi); lya_free(d_w); lya_free(d_y); lya_free(d_W); lya_free(d_mean); lya_free(d_zero); };
-  if (e != cudaSuccess) {
-    cleanup();
+  if (cov_reserve(ctx->covs, 3 * n * nb, nb, 0) != cudaSuccess)
     return lya_fail(ctx, LYA_ERR_ALLOC, "lya_covariance: device allocation failed");
-  }
+  double *d_xi = ctx->covs.rows, *d_w = d_xi + n * nb, *d_y = d_w + n * nb, *d_W = ctx->covs.bins, *d_mean = d_W + nb;
+  unsigned long long* d_zero = ctx->covs.zero;
+  cudaError_t e = cudaSuccess;
   const int blocks = ctx->num_sms * 8;
   if (from_run) {
     k_cov_from_hist<<<blocks, 256, 0, s>>>(n, nb, ctx->hist, d_xi, d_w);
@@ -221,6 +233,7 @@ extern "C" int lya_covariance(lya_ctx* ctx, int64_t n_rows, const double* xi, co
   }
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, s);
   unsigned long long nzero = 0;
+  lya_touch_pages(cov, sizeof(double) * (size_t)nb * nb);   // beside the kernels
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nzero, d_zero, sizeof(nzero), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && mean) e = cudaMemcpyAsync(mean, d_mean, sizeof(double) * nb, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && cov)
@@ -228,7 +241,6 @@ extern "C" int lya_covariance(lya_ctx* ctx, int64_t n_rows, const double* xi, co
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   float ms = 0.f;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  cleanup();
   if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_covariance: %s", cudaGetErrorString(e));
   ctx->last.kernel_ms = ms;
   if (nzero) return lya_fail(ctx, LYA_ERR_DATA, "lya_covariance: %llu bins have zero total weight", nzero);
@@ -245,20 +257,14 @@ extern "C" int lya_covariance_smooth(lya_ctx* ctx, const double* cov, double* co
     return lya_fail(ctx, LYA_ERR_STATE, "lya_covariance_smooth: no covariance from lya_covariance");
   LYA_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  double *d_cov = nullptr, *d_out = nullptr, *d_sum = nullptr;
-  unsigned long long* d_zero = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (cov) e = lya_alloc(&d_cov, (size_t)nb * nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_out, (size_t)nb * nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_sum, 2 * (size_t)nb);
-  if (e == cudaSuccess) e = lya_alloc(&d_zero, 1);
-  auto cleanup = [&]() { lya_free(d_cov); lya_free(d_out); lya_free(d_sum); lya_free(d_zero); };
-  if (e != cudaSuccess) {
-    cleanup();
+  if (cov_reserve(ctx->covs, 0, nb, (int64_t)nb * nb) != cudaSuccess)
     return lya_fail(ctx, LYA_ERR_ALLOC, "lya_covariance_smooth: device allocation failed");
-  }
-  const double* src = cov ? d_cov : ctx->cov;
-  if (cov) e = cudaMemcpyAsync(d_cov, cov, sizeof(double) * (size_t)nb * nb, cudaMemcpyHostToDevice, s);
+  // a matrix from the host is smoothed in place (k_cov_smooth reads its diagonal only, and keeps it)
+  double *d_out = ctx->covs.mat, *d_sum = ctx->covs.bins;
+  unsigned long long* d_zero = ctx->covs.zero;
+  const double* src = cov ? d_out : ctx->cov;
+  cudaError_t e = cudaSuccess;
+  if (cov) e = cudaMemcpyAsync(d_out, cov, sizeof(double) * (size_t)nb * nb, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_zero, 0, sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_sum, 0, sizeof(double) * 2 * nb, s);
   if (e == cudaSuccess) {
@@ -273,7 +279,6 @@ extern "C" int lya_covariance_smooth(lya_ctx* ctx, const double* cov, double* co
     // a zero variance leaves the covariance unsmoothed, as the reference does
     const size_t smem = sizeof(double) * 2 * (size_t)nb;
     if (smem > 227 * 1024) {
-      cleanup();
       return lya_fail(ctx, LYA_ERR_ARG, "lya_covariance_smooth: %d bins exceed the step table", nb);
     }
     e = cudaFuncSetAttribute(k_cov_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -283,13 +288,13 @@ extern "C" int lya_covariance_smooth(lya_ctx* ctx, const double* cov, double* co
       ctx->launches += 2;
       e = cudaGetLastError();
     }
+    lya_touch_pages(cov_smooth, sizeof(double) * (size_t)nb * nb);   // beside the kernels
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(cov_smooth, d_out, sizeof(double) * (size_t)nb * nb, cudaMemcpyDeviceToHost, s);
   } else if (e == cudaSuccess) {
     e = cudaMemcpyAsync(cov_smooth, src, sizeof(double) * (size_t)nb * nb, cudaMemcpyDeviceToHost, s);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cleanup();
   if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_covariance_smooth: %s", cudaGetErrorString(e));
   if (smoothed) *smoothed = nzero == 0 ? 1 : 0;
   return LYA_OK;

@@ -149,6 +149,16 @@ struct AdjScratch {
   int64_t n = 0, npad = 0, npix = 0;
 };
 
+// Scratch of lya_covariance and lya_covariance_smooth.
+struct CovScratch {
+  double* rows = nullptr;       // [3][n][nb]: xi, w, centred y
+  double* bins = nullptr;       // [2][nb]: W and mean, or the step sums and counts
+  double* mat = nullptr;        // [nb][nb] covariance from the host, smoothed in place, or the smoothed one
+  unsigned long long* zero = nullptr;   // [1]
+  int64_t cap_rows = 0, cap_mat = 0;
+  int cap_bins = 0;
+};
+
 struct lya_ctx {
   int device = 0;
   int num_sms = 148;
@@ -185,7 +195,7 @@ struct lya_ctx {
   double* get_tmp = nullptr;             // lya_corr_get's combined (hi + lo) sums, kept between calls
   int64_t get_tmp_cap = 0;
 
-  unsigned long long* stats = nullptr;   // [ST_N]
+  unsigned long long* stats = nullptr;   // [ST_N + 1]: counters, then the range's pair count (as double bits)
   int64_t* cta_begin = nullptr;          // [max ctas + 1]
   int32_t cta_cap = 0;
 
@@ -195,7 +205,7 @@ struct lya_ctx {
   int64_t cost_cap = 0;
   void* scan_tmp = nullptr;              // cub scan scratch
   size_t scan_tmp_bytes = 0;
-  unsigned long long* h_stats = nullptr; // pinned host copy: [ST_N] counters + range pair count (as double bits)
+  unsigned long long h_stats[ST_N + 1] = {};   // host copy of stats, read after the run
   cudaGraphExec_t run_graph = nullptr;   // the last run, captured
   alignas(16) unsigned char run_graph_key[512] = {};   // what it was captured for (see corr.cu)
   int64_t graph_launches = 0;            // runs replayed from the captured graph
@@ -207,7 +217,9 @@ struct lya_ctx {
   int32_t dist_shape = 0;                // lya_dist_config: launch shape of the distortion kernel
   int64_t dist_max_items = 0;            // lya_dist_config: 0 = every forest pair, else the first n
 
-  // covariance post-processing: the last covariance, kept for lya_covariance_smooth
+  // covariance post-processing: scratch kept between calls (grown, never
+  // shrunk), and the last covariance, kept for lya_covariance_smooth
+  CovScratch covs;
   double* cov = nullptr;                 // [cov_nb][cov_nb]
   int32_t cov_nb = 0;
   bool have_cov = false;
@@ -234,6 +246,14 @@ inline cudaError_t lya_alloc(T** p, size_t count) {
   if (lya_alloc_fault()) return cudaErrorMemoryAllocation;
   return cudaMalloc((void**)p, count * sizeof(T));
 }
+
+// Back the pages of a host buffer that a device copy is about to fill, with
+// several threads, keeping its contents.  A copy into pages that were never
+// written takes a fault per page inside the driver's own single-threaded copy:
+// 50 MB took 22.8 ms in 4 KB pages where the copy itself takes 2.5 ms; 8 threads
+// back them in 2.6 ms, and callers let that run beside the kernels.  Buffers
+// below 2 MB are left alone (a thread start costs as much as their faults).
+void lya_touch_pages(void* p, size_t bytes);
 
 template <typename T>
 inline void lya_free(T*& p) {

@@ -323,11 +323,11 @@ class PairEngine:
         reading loop and ``cov``/``cov_smooth`` of ``post_processing.py``).
         Returns ``(mean[nb], cov[nb, nb], cov_smooth[nb, nb] or None, smoothed)``."""
         mean = np.zeros(self.nb)
-        c = np.zeros((self.nb, self.nb))
+        c = np.empty((self.nb, self.nb))
         self._check(self.lib.lya_covariance(self.ctx, 0, None, None, N.ptr(mean), N.ptr(c)))
         if not smooth:
             return mean, c, None, False
-        cs = np.zeros_like(c)
+        cs = np.empty_like(c)
         sm = C.c_int32(0)
         self._check(self.lib.lya_covariance_smooth(self.ctx, None, N.ptr(cs), C.byref(sm)))
         return mean, c, cs, bool(sm.value)
