@@ -50,8 +50,11 @@ typedef struct {
   int32_t variant;         /* diagonal walk: 0 = default (FP32: the lean walk --
                               two diagonals per lane, bin tests on the FP32 pixel
                               coordinates -- for pairs of sorted forests with
-                              0 <= dc < 1e6, walk 2 for the others; FP64: one
-                              diagonal per lane), 1 = one diagonal per lane,
+                              0 <= dc < 1e6, walk 2 for the others; FP64: two
+                              diagonals per lane and exact bin edges for the
+                              same pairs, walk 1 for the others and for
+                              binnings whose edges do not fit shared memory),
+                              1 = one diagonal per lane,
                               2 = two diagonals per lane, 3 = same as 0 */
   int32_t run_cap;         /* longest register run of the diagonal walks before it
                               is recorded (bounds FP32 run sums): 0 = default

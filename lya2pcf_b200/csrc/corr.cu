@@ -153,6 +153,7 @@ __device__ void diagonal_band(int L1, int L2, const float4* __restrict__ P1, HiL
 // buffer into the CTA histogram with all 32 lanes when it holds 32 records or
 // more, so the long-latency FP64 shared atomics never run in a divergent branch.
 constexpr int REC = 128;   // records per warp buffer (up to 64 written per step)
+constexpr int REC_EXACT = 96;   // of the exact walk, whose edge tables need the room
 
 struct __align__(16) RecF32 {
   int bin, n;
@@ -1001,6 +1002,208 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
   }
 }
 
+// ------------------------------------------------------------------ exact walk (FP64, both forests lean)
+// The lean walk's layout with the FP64 formula's own bins: e = |dc1 - dc2| and
+// s = dc1 + dc2 in FP64 are compared with the pair's exact edges (lya_edge),
+// e >= tx[b] <=> rp bin >= b, s >= ty[b] <=> rt bin >= b, so there is no guard
+// band and no product or floor per pixel pair.  A run's state is its bin (bx, by)
+// and its edges [lo, hi) x [.., sh); a pair outside closes the run and moves the
+// bin edge by edge.  bx = np: beyond rpmax; a diagonal ends at s >= ty[nt].
+// Two diagonals per lane share the f1 pixel and take one f2 pixel per step: the
+// one-diagonal walk loads two 32-byte pixels per pair and is bound by the L1
+// data pipe (75% busy).  1.50e10 pixel pairs in 37 x 23 bins: 59 ms, the
+// one-diagonal walk 102.5 ms; 1.85e9 pairs of 200-pixel forests in 50 x 50 bins:
+// 10.8 against 17.8 ms.  Bound: issue, half of it the runs' events (128
+// registers, 16 warps per SM).
+// Tables of a warp, in shared memory (doubles): ch, sh, tx[np + 2], ty[nt + 2].
+__host__ __device__ __forceinline__ int exact_tab(int np, int nt) { return (2 + np + 2 + nt + 2 + 1) & ~1; }
+
+struct ExactRun {
+  int bx, by, k0;
+  double lo, hi, sh;
+};
+
+struct ExactAcc {
+  double aw, adw, ae, as, az;
+  __device__ __forceinline__ void zero() { aw = adw = ae = as = az = 0.0; }
+  __device__ __forceinline__ void add(const double4& a, const double4& b, double e, double s) {
+    const double w12 = __dmul_rn(a.y, b.y);
+    aw += w12;
+    adw = __fma_rn(a.z, b.z, adw);
+    ae = __fma_rn(w12, e, ae);
+    as = __fma_rn(w12, s, as);
+    az = __fma_rn(w12, __dadd_rn(a.w, b.w), az);
+  }
+};
+
+__device__ __forceinline__ double exact_e(const double4& a, const double4& b) { return fabs(__dsub_rn(a.x, b.x)); }
+__device__ __forceinline__ double exact_s(const double4& a, const double4& b) { return __dadd_rn(a.x, b.x); }
+
+struct ExactWalk {
+  const CorrParams& p;
+  const double* tx;
+  const double* ty;
+  const SmemHist& h;
+  RecF64* buf;
+  int& cnt;
+  LaneStats& st;
+  int ka_beg, kb_beg, ka_end, kb_end;
+  int kall;   // last step any lane of the warp still walks (exclusive)
+  ExactRun ra, rb;
+  ExactAcc acca, accb;
+
+  __device__ __forceinline__ void record(bool w, const ExactRun& r, const ExactAcc& acc, int k, unsigned bal, int pos) {
+    if (w) {
+      RecF64 rec;
+      rec.bin = r.bx * p.nt + r.by; rec.n = k - r.k0;
+      rec.aw = acc.aw; rec.adw = acc.adw; rec.az = acc.az;
+      rec.ax = acc.ae * tx[-2]; rec.ay = acc.as * tx[-1];   // ch, sh
+      buf[pos + __popc(bal & ((1u << (threadIdx.x & 31)) - 1u))] = rec;
+    }
+  }
+
+  // close both runs at step ka / kb for the lanes in live_*; records for in-range runs
+  __device__ __forceinline__ void close(bool live_a, bool live_b, int ka, int kb) {
+    const bool wa = live_a && ra.bx < p.np && ka > ra.k0;
+    const bool wb = live_b && rb.bx < p.np && kb > rb.k0;
+    const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
+    record(wa, ra, acca, ka, bala, cnt);
+    record(wb, rb, accb, kb, balb, cnt + __popc(bala));
+    cnt += __popc(bala) + __popc(balb);
+    if (live_a) { acca.zero(); ra.k0 = ka; }
+    if (live_b) { accb.zero(); rb.k0 = kb; }
+    if (cnt > REC_EXACT - 64) {
+      drain(buf, cnt, h, p.nb, st);
+      cnt = 0;
+    }
+  }
+
+  // Move the run to the bin of the pair (e, s); a diagonal past rtmax ends (kend = k).
+  __device__ __forceinline__ void move(ExactRun& r, double e, double s, int& kend, int k) {
+    while (e >= r.hi) { ++r.bx; r.lo = r.hi; r.hi = tx[r.bx + 1]; }
+    while (e < r.lo) { --r.bx; r.hi = r.lo; r.lo = tx[r.bx]; }
+    if (s >= r.sh) {
+      do { ++r.by; r.sh = ty[r.by + 1]; } while (s >= r.sh);
+      if (r.by >= p.nt) { r.bx = p.np; kend = k; }
+    }
+  }
+
+  // The run of a diagonal's first pair.
+  __device__ __forceinline__ void start(ExactRun& r, double e, double s, int& kend, int k) {
+    r.bx = min((int)(e * tx[-2] * p.binner_rp), p.np);
+    r.by = min((int)(s * tx[-1] * p.binner_rt), p.nt);
+    r.k0 = k;
+    r.lo = tx[r.bx]; r.hi = tx[r.bx + 1];
+    while (s < ty[r.by]) --r.by;
+    r.sh = ty[r.by + 1];
+    move(r, e, s, kend, k);
+    if (r.by >= p.nt) { r.bx = p.np; kend = k; }
+  }
+
+  __device__ __forceinline__ void step(int k, const double4& q1, const double4& qa, const double4& qb) {
+    const double ea = exact_e(q1, qa), sa = exact_s(q1, qa);
+    const double eb = exact_e(q1, qb), sb = exact_s(q1, qb);
+    bool act_a = k >= ka_beg && k < ka_end;
+    bool act_b = k >= kb_beg && k < kb_end;
+    const bool exa = act_a && (ea < ra.lo || ea >= ra.hi || sa >= ra.sh);
+    const bool exb = act_b && (eb < rb.lo || eb >= rb.hi || sb >= rb.sh);
+    if (__any_sync(FULL, exa || exb)) {
+      const bool wa = exa && ra.bx < p.np && k > ra.k0;
+      const bool wb = exb && rb.bx < p.np && k > rb.k0;
+      const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
+      record(wa, ra, acca, k, bala, cnt);
+      record(wb, rb, accb, k, balb, cnt + __popc(bala));
+      cnt += __popc(bala) + __popc(balb);
+      const int ea0 = ka_end, eb0 = kb_end;
+      if (exa) { acca.zero(); ra.k0 = k; move(ra, ea, sa, ka_end, k); }
+      if (exb) { accb.zero(); rb.k0 = k; move(rb, eb, sb, kb_end, k); }
+      if (__any_sync(FULL, ka_end != ea0 || kb_end != eb0)) {   // diagonals past rtmax shorten the walk
+        act_a = act_a && k < ka_end;
+        act_b = act_b && k < kb_end;
+        kall = min(kall, __reduce_max_sync(FULL, max(ka_end, kb_end)));
+      }
+      if (cnt > REC_EXACT - 64) {
+        drain(buf, cnt, h, p.nb, st);
+        cnt = 0;
+      }
+    }
+    if (act_a) acca.add(q1, qa, ea, sa);
+    if (act_b) accb.add(q1, qb, eb, sb);
+  }
+};
+
+__device__ void item_exact(const CorrParams& p, int64_t t, const SmemHist& h, RecF64* buf, double* tab, int& cnt,
+                           LaneStats& st) {
+  const int lane = threadIdx.x & 31;
+  const int fa = p.f1[t], fb = p.f2[t];
+  const int L1 = p.len[fa], L2 = p.len[fb];
+  if (L1 <= 0 || L2 <= 0) return;
+  const int64_t a = p.pstart[fa], b = p.pstart[fb];
+  double* tx = tab + 2;
+  double* ty = tx + p.np + 2;
+  ExactWalk W{p, tx, ty, h, buf, cnt, st};
+  double ch, sh;
+  pair_half_angles(p, fa, fb, ch, sh);
+  const double INF = inf_of<double>();
+  __syncwarp();   // every lane is done with the previous pair's tables
+  for (int k = lane; k <= p.np; k += 32) tx[k] = k == 0 ? 0.0 : lya_edge((double)k, ch, p.binner_rp);
+  for (int k = lane; k <= p.nt; k += 32) ty[k] = k == 0 ? 0.0 : lya_edge((double)k, sh, p.binner_rt);
+  if (lane == 0) { tab[0] = ch; tab[1] = sh; tx[p.np + 1] = INF; ty[p.nt + 1] = INF; }
+  __syncwarp();
+  int m_lo, m_hi;
+  {
+    const float4* __restrict__ P1 = p.pix4 + a;
+    const float4* __restrict__ P2 = p.pix4 + b;
+    const double rp_reach = ch > 0.0 ? ((double)p.np + 1e-3) / (ch * p.binner_rp) : 1e300;
+    const double rt_reach = sh > 0.0 ? ((double)p.nt + 1e-3) / (sh * p.binner_rt) : 1e300;
+    diagonal_band(L1, L2, P1, [&](int j) { return P2[j].x; }, rp_reach, rt_reach, m_lo, m_hi);
+  }
+  const int cap = p.run_cap;   // power of two, even
+  for (int mg = m_lo; mg <= m_hi; mg += 64) {
+    const int ma = mg + 2 * lane, mb = ma + 1;
+    const int ia_lo = max(0, -ma), ia_hi = (ma <= m_hi) ? min(L1, L2 - ma) : ia_lo;
+    const int ib_lo = max(0, -mb), ib_hi = (mb <= m_hi) ? min(L1, L2 - mb) : ib_lo;
+    const bool ne_a = ia_lo < ia_hi, ne_b = ib_lo < ib_hi;
+    int base = min(ne_a ? ia_lo + lane : INT_MAX, ne_b ? ib_lo + lane : INT_MAX);
+    base = __reduce_min_sync(FULL, base);
+    if (base == INT_MAX) continue;
+    W.ka_beg = ne_a ? ia_lo + lane - base : 0;
+    W.kb_beg = ne_b ? ib_lo + lane - base : 0;
+    W.ka_end = ne_a ? ia_hi + lane - base : 0;
+    W.kb_end = ne_b ? ib_hi + lane - base : 0;
+    const double4* __restrict__ A1 = p.pix8 + a + (base - lane);        // f1 pixel of step 0
+    const double4* __restrict__ A2 = p.pix8 + b + (base + mg + lane);   // f2 pixel of diagonal a
+    W.acca.zero();
+    W.accb.zero();
+    W.ra.bx = p.np; W.ra.by = 0; W.ra.k0 = 0; W.ra.lo = 0.0; W.ra.hi = INF; W.ra.sh = INF;
+    W.rb = W.ra;
+    if (ne_a) {   // each lane's first run
+      const double4 u = A1[W.ka_beg], v = A2[W.ka_beg];
+      W.start(W.ra, exact_e(u, v), exact_s(u, v), W.ka_end, W.ka_beg);
+    }
+    if (ne_b) {
+      const double4 u = A1[W.kb_beg], v = A2[W.kb_beg + 1];
+      W.start(W.rb, exact_e(u, v), exact_s(u, v), W.kb_end, W.kb_beg);
+    }
+    W.kall = __reduce_max_sync(FULL, max(W.ka_end, W.kb_end));
+    // the loads run at most 34 pixels outside a forest (LYA_MARGIN)
+    double4 q1a = A1[0], q2x = A2[0], q2y = A2[1];
+    int k = 0;
+    for (; k < W.kall; k += 2) {
+      const double4 q1b = A1[k + 1], q2z = A2[k + 2];
+      W.step(k, q1a, q2x, q2y);
+      q1a = A1[k + 2];
+      W.step(k + 1, q1b, q2y, q2z);
+      q2x = q2z;
+      q2y = A2[k + 3];
+      if (((k + 2) & (cap - 1)) == 0)   // bound the length of a run
+        W.close(k + 1 >= W.ka_beg && k + 1 < W.ka_end, k + 1 >= W.kb_beg && k + 1 < W.kb_end, k + 2, k + 2);
+    }
+    st.evaluated += (unsigned long long)(max(0, W.ka_end - W.ka_beg) + max(0, W.kb_end - W.kb_beg));
+    W.close(true, true, max(W.ka_end, W.ra.k0), max(W.kb_end, W.rb.k0));
+  }
+}
+
 // ------------------------------------------------------------------ FP64 plain (every pixel pair)
 __device__ void item_plain(const CorrParams& p, int64_t t, const SmemHist& h, LaneStats& st) {
   const int lane = threadIdx.x & 31;
@@ -1056,6 +1259,12 @@ constexpr size_t rec_bytes() {
 // p.variant names.
 enum { WALK_ANY = 0, WALK_LEAN = 1, WALK_REST = 2 };
 
+// records of a warp's buffer
+template <int KIND, int WALK>
+__host__ __device__ constexpr int rec_count() {
+  return KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_LEAN ? REC_EXACT : REC;
+}
+
 template <int KIND, int WARPS, int WALK>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1069,10 +1278,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
   // the count array keeps 8 bytes per bin so the record buffers stay 16-byte aligned
   unsigned char* bufs = reinterpret_cast<unsigned char*>(h.q + LYA_NQ * nb) + (size_t)nb * sizeof(unsigned long long);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* mybuf = bufs + (size_t)warp * REC * rec_bytes<KIND>();
-  // lean walk: per-warp state and threshold tables after the record buffers
-  LeanCtl* myctl = reinterpret_cast<LeanCtl*>(reinterpret_cast<float*>(bufs + (size_t)WARPS * REC * rec_bytes<KIND>()) +
-                                              (size_t)warp * lean_ctl_stride(p.np, p.nt));
+  constexpr int NREC = rec_count<KIND, WALK>();
+  unsigned char* mybuf = bufs + (size_t)warp * NREC * rec_bytes<KIND>();
+  // lean walk: per-warp state and threshold tables after the record buffers; exact walk: its edges
+  unsigned char* tabs = bufs + (size_t)WARPS * NREC * rec_bytes<KIND>();
+  LeanCtl* myctl = reinterpret_cast<LeanCtl*>(reinterpret_cast<float*>(tabs) + (size_t)warp * lean_ctl_stride(p.np, p.nt));
+  double* mytab = reinterpret_cast<double*>(tabs) + (size_t)warp * exact_tab(p.np, p.nt);
   __shared__ unsigned long long s_next;
   __shared__ long long s_seg_end;
   __shared__ int s_slot;
@@ -1117,6 +1328,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
         } else {
           item_diag2<TrF32, true>(p, (int64_t)t, h, reinterpret_cast<RecF32*>(mybuf), cnt, st);
         }
+      } else if (KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_LEAN) {
+        if (p.sorted[p.f1[t]] & p.sorted[p.f2[t]] & LYA_LEAN)
+          item_exact(p, (int64_t)t, h, reinterpret_cast<RecF64*>(mybuf), mytab, cnt, st);
+      } else if (KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_REST) {
+        if (!(p.sorted[p.f1[t]] & p.sorted[p.f2[t]] & LYA_LEAN))
+          item_diag<TrF64, false>(p, (int64_t)t, h, reinterpret_cast<RecF64*>(mybuf), cnt, st);
       } else if (KIND == LYA_KERNEL_FP64_DIAGONAL) {
         if (p.variant == 2) item_diag2<TrF64, false>(p, (int64_t)t, h, reinterpret_cast<RecF64*>(mybuf), cnt, st);
         else item_diag<TrF64, false>(p, (int64_t)t, h, reinterpret_cast<RecF64*>(mybuf), cnt, st);
@@ -1164,28 +1381,39 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
   }
 }
 
-template <int KIND, int WARPS>
+template <int KIND, int WARPS, int WALK>
 size_t corr_smem_bytes(const CorrParams& p, int nb) {
+  size_t tabs = 0;
+  if (KIND == LYA_KERNEL_FP32_GUARDED) tabs = (size_t)WARPS * lean_ctl_stride(p.np, p.nt) * sizeof(float);
+  if (KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_LEAN) tabs = (size_t)WARPS * exact_tab(p.np, p.nt) * sizeof(double);
   return (size_t)nb * (LYA_NQ * sizeof(double) + sizeof(unsigned long long)) +
-         (size_t)WARPS * REC * rec_bytes<KIND>() +
-         (KIND == LYA_KERNEL_FP32_GUARDED ? (size_t)WARPS * lean_ctl_stride(p.np, p.nt) * sizeof(float) : 0);
+         (size_t)WARPS * rec_count<KIND, WALK>() * rec_bytes<KIND>() + tabs;
 }
 
 template <int KIND, int WARPS, int WALK>
 cudaError_t set_corr_smem(const CorrParams& p, int nb) {
   return cudaFuncSetAttribute(k_corr<KIND, WARPS, WALK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)corr_smem_bytes<KIND, WARPS>(p, nb));
+                              (int)corr_smem_bytes<KIND, WARPS, WALK>(p, nb));
 }
 
 template <int KIND, int WARPS, int WALK>
 cudaError_t launch_corr(const CorrParams& p, int nctas, int nb, cudaStream_t s) {
-  k_corr<KIND, WARPS, WALK><<<nctas, WARPS * 32, corr_smem_bytes<KIND, WARPS>(p, nb), s>>>(p);
+  k_corr<KIND, WARPS, WALK><<<nctas, WARPS * 32, corr_smem_bytes<KIND, WARPS, WALK>(p, nb), s>>>(p);
   return cudaGetLastError();
 }
 
 // The FP32 kernel's default walk: the lean instance, plus the two-diagonal
 // instance for the pairs it skips when the catalogue has forests it cannot take.
 static bool fp32_lean_walk(int variant) { return variant == 0 || variant == 3; }
+
+// The FP64 kernel's default walk is the exact walk (and the one-diagonal walk
+// for the pairs it skips) when its records and edge tables fit the shared memory
+// beside the histogram: every binning the one-diagonal walk fits with np + nt up
+// to 180, and 2,500 bins with np + nt up to 290.
+static bool fp64_exact_walk(const CorrParams& p, int nb) {
+  return p.variant == 0 &&
+         corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, nb) <= 226 * 1024;
+}
 
 // ------------------------------------------------------------------ CTA ranges
 __global__ void k_item_cost(int64_t n, const int32_t* __restrict__ f1, const int32_t* __restrict__ f2,
@@ -1287,6 +1515,9 @@ static cudaError_t enqueue_run(lya_ctx* ctx, const RunGraphKey& k, double* d_ran
       if (e == cudaSuccess && k.rest_pass) e = launch_corr<LYA_KERNEL_FP32_GUARDED, 16, WALK_REST>(p, k.nctas, k.nb, s);
     } else if (k.kind == LYA_KERNEL_FP32_GUARDED) {
       e = launch_corr<LYA_KERNEL_FP32_GUARDED, 16, WALK_ANY>(p, k.nctas, k.nb, s);
+    } else if (k.kind == LYA_KERNEL_FP64_DIAGONAL && fp64_exact_walk(p, k.nb)) {
+      e = launch_corr<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, k.nctas, k.nb, s);
+      if (e == cudaSuccess && k.rest_pass) e = launch_corr<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, k.nctas, k.nb, s);
     } else if (k.kind == LYA_KERNEL_FP64_DIAGONAL) {
       e = launch_corr<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_ANY>(p, k.nctas, k.nb, s);
     } else {
@@ -1377,7 +1608,9 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
   p.hist = ctx->hist; p.counts = ctx->counts; p.stats = ctx->stats;
   key.kind = kind; key.nctas = nctas; key.nslots = nslots; key.nb = nb; key.n_items = n;
   key.slot_begin = o->slot_begin; key.slot_end = o->slot_end;
-  key.rest_pass = (kind == LYA_KERNEL_FP32_GUARDED && fp32_lean_walk(o->variant) && ctx->cat.n_not_lean > 0) ? 1 : 0;
+  const bool exact = kind == LYA_KERNEL_FP64_DIAGONAL && fp64_exact_walk(p, nb);
+  const bool skips = exact || (kind == LYA_KERNEL_FP32_GUARDED && fp32_lean_walk(o->variant));
+  key.rest_pass = skips && ctx->cat.n_not_lean > 0 ? 1 : 0;
   key.cost = ctx->cost; key.scan_tmp = ctx->scan_tmp; key.scan_bytes = scan_bytes;
 
   // shared-memory limit of the pair kernel: set outside any capture
@@ -1387,6 +1620,9 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
       e = set_corr_smem<LYA_KERNEL_FP32_GUARDED, 16, WALK_LEAN>(p, nb);
       if (e == cudaSuccess) e = set_corr_smem<LYA_KERNEL_FP32_GUARDED, 16, WALK_REST>(p, nb);
       if (e == cudaSuccess) e = set_corr_smem<LYA_KERNEL_FP32_GUARDED, 16, WALK_ANY>(p, nb);
+    } else if (exact) {
+      e = set_corr_smem<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, nb);
+      if (e == cudaSuccess && key.rest_pass) e = set_corr_smem<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, nb);
     } else if (kind == LYA_KERNEL_FP64_DIAGONAL) {
       e = set_corr_smem<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_ANY>(p, nb);
     } else {

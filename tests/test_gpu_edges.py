@@ -90,3 +90,26 @@ def test_distortion_edges(np_, nt, step, unsorted):
     Do, Wo = O.distortion(fs, f1, f2, np_=np_, nt=nt)
     np.testing.assert_allclose(W, Wo, rtol=1e-12, atol=1e-12 * np.abs(Wo).max())
     assert np.abs(D - Do).max() <= 1e-10 * np.abs(Do).max() and np.abs(Do).max() > 0
+
+
+@pytest.mark.parametrize('np_,nt,step,unsorted', [
+    (50, 50, 2.0, False), (50, 50, 2.0, True), (50, 50, 9.0, False), (200, 12, 2.0, False), (12, 200, 2.0, False),
+    (1, 1, 2.0, False), (300, 8, 2.0, False),
+    (600, 4, 2.0, False)])   # the last: edge tables beyond the shared memory, the one-diagonal walk
+def test_fp64_walk_edges(np_, nt, step, unsorted):
+    """FP64 kernel against the oracle: counts equal, sums to 1e-12 (DW to 1e-12
+    of the sum of the moduli), as in the other FP64 tests."""
+    fs = ragged(step, unsorted)
+    f1, f2 = all_pairs(fs)
+    slot_start = np.searchsorted(fs.pix[f1], np.arange(fs.pix[-1] + 2))
+    hist, cnt = O.corr(fs, f1, f2, slot_start, np_=np_, nt=nt)
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        for run_cap in (0, 8):
+            eng.run(kernel=N.KERNEL_FP64_DIAGONAL, run_cap=run_cap)
+            h, c = eng.histograms()
+            assert np.array_equal(c, cnt) and cnt.sum() > 0
+            for q in (N.Q_W, N.Q_DW, N.Q_RP, N.Q_RT, N.Q_Z):
+                scale = hist[:, O.Q_DWABS if q == N.Q_DW else q]
+                assert np.all(np.abs(h[:, q] - hist[:, q]) <= 1e-12 * scale), q
