@@ -76,8 +76,11 @@ struct CorrParams {
   unsigned long long* stats;    // [ST_N]
 };
 
+// Statistics of a lane within one owner slot's segment, added to the CTA's
+// 64-bit sums at its end (64-bit lane sums would hold eight registers through
+// the walks).
 struct LaneStats {
-  unsigned long long evaluated = 0, recheck = 0, runs = 0, inrange = 0;
+  unsigned evaluated = 0, recheck = 0, runs = 0, inrange = 0;
 };
 
 // Shared-memory histogram of the slot being accumulated.
@@ -153,7 +156,7 @@ __device__ void diagonal_band(int L1, int L2, const float4* __restrict__ P1, HiL
 // buffer into the CTA histogram with all 32 lanes when it holds 32 records or
 // more, so the long-latency FP64 shared atomics never run in a divergent branch.
 constexpr int REC = 128;   // records per warp buffer (up to 64 written per step)
-constexpr int REC_EXACT = 96;   // of the exact walk, whose edge tables need the room
+constexpr int REC_EXACT = 80;   // of the exact walk, whose edge tables need the room
 
 struct __align__(16) RecF32 {
   int bin, n;
@@ -170,12 +173,13 @@ __device__ __forceinline__ void drain(Rec* buf, int cnt, const SmemHist& h, int 
   __syncwarp();
   for (int k = lane; k < cnt; k += 32) {
     const Rec r = buf[k];
-    if ((unsigned)r.bin >= (unsigned)nb || r.n <= 0) {   // never written by a correct walk: report, skip
+    if (r.n == 0) continue;   // a run beyond rpmax (exact walk)
+    if ((unsigned)r.bin >= (unsigned)nb || r.n < 0) {   // never written by a correct walk: report, skip
       atomicOr(h.err, 1ull);
       continue;
     }
     st.runs++;
-    st.inrange += (unsigned long long)r.n;
+    st.inrange += (unsigned)r.n;
     atomicAdd(&h.q[0 * nb + r.bin], (double)r.aw);
     atomicAdd(&h.q[1 * nb + r.bin], (double)r.adw);
     atomicAdd(&h.q[2 * nb + r.bin], (double)r.ax);
@@ -444,7 +448,7 @@ __device__ void item_diag(const CorrParams& p, int64_t t, const SmemHist& h, typ
           if (__all_sync(FULL, k + 1 >= stop)) break;
         }
       }
-      st.evaluated += (unsigned long long)max(0, min(stop, k_end) - k_beg);
+      st.evaluated += (unsigned)max(0, min(stop, k_end) - k_beg);
       const int kfin = min(stop, k_end);
       close_runs<Tr>(true, r, acc, max(kfin, r.k0), nt, buf, cnt, lt, st);
       if (cnt > REC - 32) {
@@ -649,7 +653,7 @@ __device__ void item_diag2(const CorrParams& p, int64_t t, const SmemHist& h, ty
       }
     }
     const int kfa = min(W.stop_a, k_end), kfb = min(W.stop_b, k_end);
-    st.evaluated += (unsigned long long)(max(0, kfa - W.ka_beg) + max(0, kfb - W.kb_beg));
+    st.evaluated += (unsigned)(max(0, kfa - W.ka_beg) + max(0, kfb - W.kb_beg));
     W.close(true, true, max(kfa, W.ra.k0), max(kfb, W.rb.k0));
   }
 }
@@ -682,28 +686,38 @@ __device__ void item_diag2(const CorrParams& p, int64_t t, const SmemHist& h, ty
 // rotate without copies.
 // Per-warp state of the forest pair being walked, in shared memory (read on
 // the rare paths only, so the walk's registers hold just the runs, the sums and
-// the pixels); the threshold tables follow it: tlo[np], thi[np], slo[nt], shi[nt].
+// the pixels); the threshold tables follow it: (tlo, thi) of rp bins 0 .. np and
+// (slo, shi) of rt bins 0 .. nt, bin np and nt being "beyond the last edge".
 struct __align__(16) LeanCtl {
   double ch, sh;
   const double4* d1;     // FP64 pixels of f1 (i = 0)
   const double4* d2;     // FP64 pixels of f2 (j = 0)
-  float tout, scut;      // e >= tout: beyond rpmax;  s >= scut: beyond rtmax
   float cxf, cyf;        // FP32 copies of cx, cy: candidate bins and record scaling
   int base, mg;          // current pass: f1 pixel i = base + k - lane, f2 pixel j = base + mg + lane + k
-  int pad0, pad1;
 };
 constexpr int LEAN_CTL_FLOATS = (int)(sizeof(LeanCtl) / sizeof(float));
 // floats per warp: the state and the tables, rounded to keep the next warp's state 16-byte aligned
 __host__ __device__ __forceinline__ int lean_ctl_stride(int np, int nt) {
-  return LEAN_CTL_FLOATS + ((2 * (np + nt) + 3) & ~3);
+  return LEAN_CTL_FLOATS + ((2 * (np + 1 + nt + 1) + 3) & ~3);
 }
 
-__device__ __forceinline__ float* lean_tab(LeanCtl* c) { return reinterpret_cast<float*>(c + 1); }
+__device__ __forceinline__ const float2* lean_x(const LeanCtl* c) { return reinterpret_cast<const float2*>(c + 1); }
+__device__ __forceinline__ const float2* lean_y(const LeanCtl* c, int np) { return lean_x(c) + np + 1; }
 
+// Run state: bin (bx, by), bx = np beyond rpmax; interval [lo, hi) x [.., sh);
+// first step k0.
 struct LeanRun {
   int bx, by, k0;
-  float tlo, thi, shi;
+  float lo, hi, sh;
 };
+
+// A run's record: bin and length packed (4096 bins, runs of at most 1024 pairs),
+// the sums of w12 e and w12 s not yet scaled to bin units.
+struct __align__(8) RecLean {
+  unsigned key;   // n << 12 | bin
+  float aw, adw, ae, as, az;
+};
+static_assert(LYA_MAX_BINS <= 4096, "a record's bin has 12 bits");
 
 struct LeanAcc {
   float aw, adw, ae, as, az;
@@ -721,34 +735,24 @@ struct LeanAcc {
 __device__ __forceinline__ float lean_e(const float4& a, const float4& b) { return fabsf((a.x - b.x) + (a.y - b.y)); }
 __device__ __forceinline__ float lean_s(const float4& a, const float4& b) { return a.x + b.x; }
 
-// true when the pair (e, s) lies outside the run's interval (NaN-safe form)
-__device__ __forceinline__ bool lean_out(const LeanRun& r, float e, float s) {
-  return !(e >= r.tlo) || !(e < r.thi) || !(s < r.shi);
-}
-
 // Per-forest-pair state and threshold tables of one warp.
 __device__ __forceinline__ void lean_setup(LeanCtl* c, double ch, double sh, const double4* d1, const double4* d2,
                                            const CorrParams& p) {
   const int lane = threadIdx.x & 31;
+  const float INF = __int_as_float(0x7f800000);
   __syncwarp();   // every lane is done with the previous forest pair's state
   const double cx = __dmul_rn(ch, p.binner_rp), cy = __dmul_rn(sh, p.binner_rt);
   const double gx = (double)p.gx, gy = (double)p.gy;
-  float* tlo = lean_tab(c);
-  float* thi = tlo + p.np;
-  float* slo = thi + p.np;
-  float* shi = slo + p.nt;
-  for (int b = lane; b < p.np; b += 32) {
-    tlo[b] = b == 0 ? -1.0f : __double2float_ru(__ddiv_ru((double)b + gx, cx));
-    thi[b] = __double2float_rd(__ddiv_rd((double)(b + 1) - gx, cx));
-  }
-  for (int b = lane; b < p.nt; b += 32) {
-    slo[b] = b == 0 ? -1.0f : __double2float_ru(__ddiv_ru((double)b + gy, cy));
-    shi[b] = __double2float_rd(__ddiv_rd((double)(b + 1) - gy, cy));
-  }
+  float2* x = const_cast<float2*>(lean_x(c));
+  float2* y = const_cast<float2*>(lean_y(c, p.np));
+  for (int b = lane; b <= p.np; b += 32)
+    x[b] = make_float2(b == 0 ? -1.0f : __double2float_ru(__ddiv_ru((double)b + gx, cx)),
+                       b == p.np ? INF : __double2float_rd(__ddiv_rd((double)(b + 1) - gx, cx)));
+  for (int b = lane; b <= p.nt; b += 32)
+    y[b] = make_float2(b == 0 ? -1.0f : __double2float_ru(__ddiv_ru((double)b + gy, cy)),
+                       b == p.nt ? INF : __double2float_rd(__ddiv_rd((double)(b + 1) - gy, cy)));
   if (lane == 0) {
     c->ch = ch; c->sh = sh; c->d1 = d1; c->d2 = d2;
-    c->tout = __double2float_ru(__ddiv_ru((double)p.np + gx, cx));
-    c->scut = __double2float_ru(__ddiv_ru((double)p.nt + gy, cy));
     c->cxf = __double2float_rn(cx);
     c->cyf = __double2float_rn(cy);
   }
@@ -761,25 +765,22 @@ __device__ __forceinline__ void lean_setup(LeanCtl* c, double ch, double sh, con
 __device__ __forceinline__ void lean_classify(const CorrParams& p, const LeanCtl* c, LeanRun& r, float e, float s,
                                            int& kend, int k, int dm, LaneStats& st) {
   const float INF = __int_as_float(0x7f800000);
-  const float* tlo = lean_tab(const_cast<LeanCtl*>(c));
-  const float* thi = tlo + p.np;
-  const float* slo = thi + p.np;
-  const float* shi = slo + p.nt;
-  const float scut = c->scut, tout = c->tout;
-  if (!(s < scut)) {   // past rtmax for good (s only grows): the diagonal is done
+  const float2* X = lean_x(c);
+  const float2* Y = lean_y(c, p.np);
+  if (!(s < Y[p.nt].x)) {   // past rtmax for good (s only grows): the diagonal is done
     kend = k;
-    r.bx = -1; r.by = -1; r.tlo = -INF; r.thi = INF; r.shi = INF;
+    r.bx = p.np; r.by = p.nt; r.lo = -INF; r.hi = INF; r.sh = INF;
     return;
   }
-  if (e >= tout) {     // beyond rpmax; |dc1-dc2| may shrink again
-    r.bx = -1; r.by = -1; r.tlo = tout; r.thi = INF; r.shi = scut;
+  if (e >= X[p.np].x) {     // beyond rpmax; |dc1-dc2| may shrink again
+    r.bx = p.np; r.by = min((int)(s * c->cyf), p.nt - 1); r.lo = X[p.np].x; r.hi = INF; r.sh = Y[p.nt].x;
     return;
   }
-  const int cbx = min((int)(e * c->cxf), p.np - 1);
-  const int cby = min((int)(s * c->cyf), p.nt - 1);
-  const float tl = tlo[cbx], th = thi[cbx], sl = slo[cby], su = shi[cby];
-  if (e >= tl && e < th && s >= sl && s < su) {
-    r.bx = cbx; r.by = cby; r.tlo = tl; r.thi = th; r.shi = su;
+  r.bx = min((int)(e * c->cxf), p.np - 1);
+  r.by = min((int)(s * c->cyf), p.nt - 1);
+  const float2 x = X[r.bx], y = Y[r.by];
+  if (e >= x.x && e < x.y && s >= y.x && s < y.y) {
+    r.lo = x.x; r.hi = x.y; r.sh = y.y;
     return;
   }
   // guard band (or an FP32 candidate one bin off): the reference FP64 formula
@@ -788,79 +789,90 @@ __device__ __forceinline__ void lean_classify(const CorrParams& p, const LeanCtl
   const int i = c->base - lane + k, j = c->base + c->mg + lane + k + dm;
   double rp, rt;
   const int b = bin_fp64(p, c->d1[i].x, c->d2[j].x, c->ch, c->sh, rp, rt);
-  if (b >= 0) { r.bx = b / p.nt; r.by = b - r.bx * p.nt; } else { r.bx = -1; r.by = -1; }
-  r.tlo = INF; r.thi = -INF; r.shi = -INF;
+  if (b >= 0) { r.bx = b / p.nt; r.by = b - r.bx * p.nt; } else r.bx = p.np;
+  r.lo = INF; r.hi = -INF; r.sh = INF;
   st.recheck++;
 }
 
-// Move the run to the adjacent bin the pair (e, s) lies in, when one rp or one
-// rt edge was crossed; false when a full classification is needed.
-__device__ __forceinline__ bool lean_shift(const CorrParams& p, const LeanCtl* c, LeanRun& r, float e, float s) {
-  const float INF = __int_as_float(0x7f800000);
-  if (r.bx < 0) return false;
-  const bool xo = !(e >= r.tlo) || !(e < r.thi);
-  const bool yo = !(s < r.shi);
-  if (xo == yo) return false;
-  const float* tlo = lean_tab(const_cast<LeanCtl*>(c));
-  if (xo) {
-    const int nbx = e >= r.thi ? r.bx + 1 : r.bx - 1;
-    if (nbx >= p.np) {
-      const float tout = c->tout;
-      if (!(e >= tout)) return false;
-      r.bx = -1; r.by = -1; r.tlo = tout; r.thi = INF; r.shi = c->scut;
-      return true;
-    }
-    if (nbx < 0) return false;
-    const float tl = tlo[nbx], th = tlo[p.np + nbx];
-    if (!(e >= tl && e < th)) return false;
-    r.bx = nbx; r.tlo = tl; r.thi = th;
-    return true;
-  }
-  const int nby = r.by + 1;
-  if (nby >= p.nt) return false;
-  const float sl = tlo[2 * p.np + nby], su = tlo[2 * p.np + p.nt + nby];
-  if (!(s >= sl && s < su)) return false;
-  r.by = nby; r.shi = su;
+// Move the run to the bin of the pair (e, s) when it is the same bin or the next
+// one in rp and in rt; false when a full classification is needed.  The bins'
+// bounds are read before they are known to be the right ones: no branch.
+__device__ __forceinline__ bool lean_move(const CorrParams& p, const LeanCtl* c, LeanRun& r, float e, float s) {
+  const int nx = r.bx + (e >= r.hi ? 1 : 0) - (e < r.lo ? 1 : 0);
+  const int ny = r.by + (s >= r.sh ? 1 : 0);
+  const float2 x = lean_x(c)[nx], y = lean_y(c, p.np)[ny];
+  if (!(e >= x.x && e < x.y && s >= y.x && s < y.y && ny < p.nt)) return false;
+  r.bx = nx; r.by = ny; r.lo = x.x; r.hi = x.y; r.sh = y.y;
   return true;
+}
+
+// Add the warp's records to the CTA's histogram (all lanes), scaled to bin units.
+__device__ __forceinline__ void lean_drain(const RecLean* buf, int cnt, const LeanCtl* c, const SmemHist& h, int nb,
+                                           LaneStats& st) {
+  __syncwarp();
+  const float cxf = c->cxf, cyf = c->cyf;
+  for (int k = threadIdx.x & 31; k < cnt; k += 32) {
+    const RecLean r = buf[k];
+    const unsigned bin = r.key & 4095u, n = r.key >> 12;
+    if (n == 0) continue;
+    if (bin >= (unsigned)nb) {   // never written by a correct walk: report, skip
+      atomicOr(h.err, 1ull);
+      continue;
+    }
+    st.runs++;
+    st.inrange += n;
+    atomicAdd(&h.q[0 * nb + bin], (double)r.aw);
+    atomicAdd(&h.q[1 * nb + bin], (double)r.adw);
+    atomicAdd(&h.q[2 * nb + bin], (double)(r.ae * cxf));
+    atomicAdd(&h.q[3 * nb + bin], (double)(r.as * cyf));
+    atomicAdd(&h.q[4 * nb + bin], (double)r.az);
+    count_pairs(h, (int)bin, n);
+  }
+  __syncwarp();
 }
 
 struct LeanWalk {
   const CorrParams& p;
   LeanCtl* c;
   const SmemHist& h;
-  RecF32* buf;
-  int& cnt;
+  RecLean* buf;
   LaneStats& st;
+  int cnt;    // records pending in the warp's buffer (warp-uniform)
   int ka_beg, kb_beg, ka_end, kb_end;
   int kall;   // last step any lane of the warp still walks (exclusive)
   LeanRun ra, rb;
   LeanAcc acca, accb;
 
-  __device__ __forceinline__ void record(bool w, const LeanRun& r, const LeanAcc& acc, int k, unsigned bal, int pos) {
+  __device__ __forceinline__ void record(bool w, const LeanRun& r, const LeanAcc& acc, int k, int pos) {
     if (w) {
-      const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
-      RecF32 rec;
-      rec.bin = r.bx * p.nt + r.by; rec.n = k - r.k0;
-      rec.aw = acc.aw; rec.adw = acc.adw; rec.ax = acc.ae * c->cxf; rec.ay = acc.as * c->cyf; rec.az = acc.az;
-      rec.pad = 0.f;
-      buf[pos + __popc(bal & lt)] = rec;
+      RecLean rec;
+      rec.key = (r.bx < p.np ? (unsigned)(k - r.k0) << 12 : 0u) | (unsigned)(r.bx * p.nt + r.by);
+      rec.aw = acc.aw; rec.adw = acc.adw; rec.ae = acc.ae; rec.as = acc.as; rec.az = acc.az;
+      buf[pos] = rec;
     }
+  }
+
+  // records of the runs in w_a, w_b, which end at steps ka, kb
+  __device__ __forceinline__ void records(bool w_a, bool w_b, int ka, int kb) {
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    const unsigned bala = __ballot_sync(FULL, w_a), balb = __ballot_sync(FULL, w_b);
+    record(w_a, ra, acca, ka, cnt + __popc(bala & lt));
+    cnt += __popc(bala);
+    record(w_b, rb, accb, kb, cnt + __popc(balb & lt));
+    cnt += __popc(balb);
+  }
+
+  __device__ __forceinline__ void flush() {
+    lean_drain(buf, cnt, c, h, p.nb, st);
+    cnt = 0;
   }
 
   // close both runs at step ka / kb for the lanes in live_*; records for in-range runs
   __device__ __forceinline__ void close(bool live_a, bool live_b, int ka, int kb) {
-    const bool wa = live_a && ra.bx >= 0 && ka > ra.k0;
-    const bool wb = live_b && rb.bx >= 0 && kb > rb.k0;
-    const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
-    record(wa, ra, acca, ka, bala, cnt);
-    record(wb, rb, accb, kb, balb, cnt + __popc(bala));
-    cnt += __popc(bala) + __popc(balb);
+    records(live_a && ra.bx < p.np && ka > ra.k0, live_b && rb.bx < p.np && kb > rb.k0, ka, kb);
     if (live_a) { acca.zero(); ra.k0 = ka; }
     if (live_b) { accb.zero(); rb.k0 = kb; }
-    if (cnt > REC - 64) {
-      drain(buf, cnt, h, p.nb, st);
-      cnt = 0;
-    }
+    if (cnt > REC - 64) flush();
   }
 
   // One step: pair a = (q1, qa), pair b = (q1, qb), with the warp's events.
@@ -873,40 +885,37 @@ struct LeanWalk {
     const float eb = lean_e(q1, qb), sb = lean_s(q1, qb);
     bool act_a = k >= ka_beg && k < ka_end;
     bool act_b = k >= kb_beg && k < kb_end;
-    const bool exa = act_a && lean_out(ra, ea, sa);
-    const bool exb = act_b && lean_out(rb, eb, sb);
-    if (__any_sync(FULL, exa || exb)) {
-      const bool wa = exa && ra.bx >= 0 && k > ra.k0;
-      const bool wb = exb && rb.bx >= 0 && k > rb.k0;
-      const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
-      record(wa, ra, acca, k, bala, cnt);
-      record(wb, rb, accb, k, balb, cnt + __popc(bala));
-      cnt += __popc(bala) + __popc(balb);
-      const bool fa = exa && !lean_shift(p, c, ra, ea, sa);
-      const bool fb = exb && !lean_shift(p, c, rb, eb, sb);
-      if (exa) { acca.zero(); ra.k0 = k; }
-      if (exb) { accb.zero(); rb.k0 = k; }
+    const bool exa = act_a && (ea < ra.lo || ea >= ra.hi || sa >= ra.sh);
+    const bool exb = act_b && (eb < rb.lo || eb >= rb.hi || sb >= rb.sh);
+    const unsigned eva = __ballot_sync(FULL, exa), evb = __ballot_sync(FULL, exb);
+    if (eva | evb) {
+      const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+      bool fa = false, fb = false;
+      if (eva) {
+        record(exa, ra, acca, k, cnt + __popc(eva & lt));
+        cnt += __popc(eva);
+        if (exa) { acca.zero(); ra.k0 = k; fa = !lean_move(p, c, ra, ea, sa); }
+      }
+      if (evb) {
+        record(exb, rb, accb, k, cnt + __popc(evb & lt));
+        cnt += __popc(evb);
+        if (exb) { accb.zero(); rb.k0 = k; fb = !lean_move(p, c, rb, eb, sb); }
+      }
       if (__any_sync(FULL, fa || fb)) {
         if (fa) lean_classify(p, c, ra, ea, sa, ka_end, k, 0, st);
         if (fb) lean_classify(p, c, rb, eb, sb, kb_end, k, 1, st);
         act_a = act_a && k < ka_end;
         act_b = act_b && k < kb_end;
-        int ke = max(ka_end, kb_end);   // diagonals past rtmax shorten the walk
-        ke = __reduce_max_sync(FULL, ke);
-        kall = min(kall, ke);
+        kall = min(kall, __reduce_max_sync(FULL, max(ka_end, kb_end)));   // diagonals past rtmax shorten the walk
       }
-      if (cnt > REC - 64) {
-        drain(buf, cnt, h, p.nb, st);
-        cnt = 0;
-      }
+      if (cnt > REC - 64) flush();
     }
     if (act_a) acca.add(q1, z1, qa, za, ea, sa);
     if (act_b) accb.add(q1, z1, qb, zb, eb, sb);
   }
 };
 
-__device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, RecF32* buf, LeanCtl* ctl, int& cnt,
-                          LaneStats& st) {
+__device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, RecLean* buf, LeanCtl* ctl, LaneStats& st) {
   const int lane = threadIdx.x & 31;
   const int fa = p.f1[t], fb = p.f2[t];
   const int L1 = p.len[fa], L2 = p.len[fb];
@@ -924,7 +933,8 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
     const double rt_reach = sh > 0.0 ? ((double)p.nt + slack) / (sh * p.binner_rt) : 1e300;
     diagonal_band(L1, L2, P1, [&](int j) { return P2[j].x; }, rp_reach, rt_reach, m_lo, m_hi);
   }
-  LeanWalk W{p, ctl, h, buf, cnt, st};
+  LeanWalk W{p, ctl, h, buf, st};
+  W.cnt = 0;
   const int cap = p.run_cap;   // power of two, even
   for (int mg = m_lo; mg <= m_hi; mg += 64) {
     const int ma = mg + 2 * lane, mb = ma + 1;
@@ -955,7 +965,7 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
     W.accb.zero();
     {
       const float INF = __int_as_float(0x7f800000);
-      W.ra.bx = -1; W.ra.by = -1; W.ra.tlo = INF; W.ra.thi = -INF; W.ra.shi = -INF;
+      W.ra.bx = p.np; W.ra.by = 0; W.ra.lo = -INF; W.ra.hi = INF; W.ra.sh = INF;
       W.rb = W.ra;
       W.ra.k0 = W.ka_beg;
       W.rb.k0 = W.kb_beg;
@@ -997,9 +1007,10 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
       }
     }
     const int kfa = min(W.ka_end, k_end), kfb = min(W.kb_end, k_end);
-    st.evaluated += (unsigned long long)(max(0, kfa - W.ka_beg) + max(0, kfb - W.kb_beg));
+    st.evaluated += (unsigned)(max(0, kfa - W.ka_beg) + max(0, kfb - W.kb_beg));
     W.close(true, true, max(kfa, W.ra.k0), max(kfb, W.rb.k0));
   }
+  W.flush();   // the scaling is this pair's
 }
 
 // ------------------------------------------------------------------ exact walk (FP64, both forests lean)
@@ -1017,6 +1028,26 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
 // registers, 16 warps per SM).
 // Tables of a warp, in shared memory (doubles): ch, sh, tx[np + 2], ty[nt + 2].
 __host__ __device__ __forceinline__ int exact_tab(int np, int nt) { return (2 + np + 2 + nt + 2 + 1) & ~1; }
+
+// Lanes of a pass of the exact walk: the last pass over a forest pair's diagonals
+// has fewer than 64.  When 32 or fewer are left, the lanes are dealt out several
+// times over, each copy walking its own segment of the steps (an even number):
+// nl lanes hold the diagonals, copies = 32 / nl.  A lane then reads at most 50
+// pixels past the end of a forest (LYA_MARGIN).  The runs of a split diagonal are
+// cut once more, which FP64 sums do not feel; the FP32 walk, whose sums depend on
+// where runs are cut, keeps its lanes as they are (cut at its run caps only, the
+// split gained it nothing).
+struct PassLanes {
+  int nl, copies;
+};
+__device__ __forceinline__ PassLanes pass_lanes(int diagonals) {
+  PassLanes g = {32, 1};
+  while (g.nl > 4 && diagonals <= g.nl) { g.nl >>= 1; g.copies <<= 1; }
+  return g;
+}
+__device__ __forceinline__ int pass_segment(const PassLanes& g, int steps) {
+  return g.copies == 1 ? steps : 2 * ((steps + 2 * g.copies - 1) / (2 * g.copies));
+}
 
 struct ExactRun {
   int bx, by, k0;
@@ -1052,10 +1083,10 @@ struct ExactWalk {
   ExactRun ra, rb;
   ExactAcc acca, accb;
 
-  __device__ __forceinline__ void record(bool w, const ExactRun& r, const ExactAcc& acc, int k, unsigned bal, int pos) {
+  __device__ __forceinline__ void record(bool w, const ExactRun& r, const ExactAcc& acc, int n, unsigned bal, int pos) {
     if (w) {
       RecF64 rec;
-      rec.bin = r.bx * p.nt + r.by; rec.n = k - r.k0;
+      rec.bin = r.bx * p.nt + r.by; rec.n = n;
       rec.aw = acc.aw; rec.adw = acc.adw; rec.az = acc.az;
       rec.ax = acc.ae * tx[-2]; rec.ay = acc.as * tx[-1];   // ch, sh
       buf[pos + __popc(bal & ((1u << (threadIdx.x & 31)) - 1u))] = rec;
@@ -1067,8 +1098,8 @@ struct ExactWalk {
     const bool wa = live_a && ra.bx < p.np && ka > ra.k0;
     const bool wb = live_b && rb.bx < p.np && kb > rb.k0;
     const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
-    record(wa, ra, acca, ka, bala, cnt);
-    record(wb, rb, accb, kb, balb, cnt + __popc(bala));
+    record(wa, ra, acca, ka - ra.k0, bala, cnt);
+    record(wb, rb, accb, kb - rb.k0, balb, cnt + __popc(bala));
     cnt += __popc(bala) + __popc(balb);
     if (live_a) { acca.zero(); ra.k0 = ka; }
     if (live_b) { accb.zero(); rb.k0 = kb; }
@@ -1107,16 +1138,19 @@ struct ExactWalk {
     bool act_b = k >= kb_beg && k < kb_end;
     const bool exa = act_a && (ea < ra.lo || ea >= ra.hi || sa >= ra.sh);
     const bool exb = act_b && (eb < rb.lo || eb >= rb.hi || sb >= rb.sh);
-    if (__any_sync(FULL, exa || exb)) {
-      const bool wa = exa && ra.bx < p.np && k > ra.k0;
-      const bool wb = exb && rb.bx < p.np && k > rb.k0;
-      const unsigned bala = __ballot_sync(FULL, wa), balb = __ballot_sync(FULL, wb);
-      record(wa, ra, acca, k, bala, cnt);
-      record(wb, rb, accb, k, balb, cnt + __popc(bala));
-      cnt += __popc(bala) + __popc(balb);
+    const unsigned eva = __ballot_sync(FULL, exa), evb = __ballot_sync(FULL, exb);
+    if (eva | evb) {   // runs beyond rpmax are recorded with n = 0
       const int ea0 = ka_end, eb0 = kb_end;
-      if (exa) { acca.zero(); ra.k0 = k; move(ra, ea, sa, ka_end, k); }
-      if (exb) { accb.zero(); rb.k0 = k; move(rb, eb, sb, kb_end, k); }
+      if (eva) {
+        record(exa, ra, acca, ra.bx < p.np ? k - ra.k0 : 0, eva, cnt);
+        cnt += __popc(eva);
+        if (exa) { acca.zero(); ra.k0 = k; move(ra, ea, sa, ka_end, k); }
+      }
+      if (evb) {
+        record(exb, rb, accb, rb.bx < p.np ? k - rb.k0 : 0, evb, cnt);
+        cnt += __popc(evb);
+        if (exb) { accb.zero(); rb.k0 = k; move(rb, eb, sb, kb_end, k); }
+      }
       if (__any_sync(FULL, ka_end != ea0 || kb_end != eb0)) {   // diagonals past rtmax shorten the walk
         act_a = act_a && k < ka_end;
         act_b = act_b && k < kb_end;
@@ -1160,19 +1194,27 @@ __device__ void item_exact(const CorrParams& p, int64_t t, const SmemHist& h, Re
   }
   const int cap = p.run_cap;   // power of two, even
   for (int mg = m_lo; mg <= m_hi; mg += 64) {
-    const int ma = mg + 2 * lane, mb = ma + 1;
+    const PassLanes g = pass_lanes(m_hi - mg + 1);
+    const int gl = lane & (g.nl - 1);
+    const int ma = mg + 2 * gl, mb = ma + 1;
     const int ia_lo = max(0, -ma), ia_hi = (ma <= m_hi) ? min(L1, L2 - ma) : ia_lo;
     const int ib_lo = max(0, -mb), ib_hi = (mb <= m_hi) ? min(L1, L2 - mb) : ib_lo;
-    const bool ne_a = ia_lo < ia_hi, ne_b = ib_lo < ib_hi;
-    int base = min(ne_a ? ia_lo + lane : INT_MAX, ne_b ? ib_lo + lane : INT_MAX);
+    int base = min(ia_lo < ia_hi ? ia_lo + gl : INT_MAX, ib_lo < ib_hi ? ib_lo + gl : INT_MAX);
     base = __reduce_min_sync(FULL, base);
     if (base == INT_MAX) continue;
-    W.ka_beg = ne_a ? ia_lo + lane - base : 0;
-    W.kb_beg = ne_b ? ib_lo + lane - base : 0;
-    W.ka_end = ne_a ? ia_hi + lane - base : 0;
-    W.kb_end = ne_b ? ib_hi + lane - base : 0;
-    const double4* __restrict__ A1 = p.pix8 + a + (base - lane);        // f1 pixel of step 0
-    const double4* __restrict__ A2 = p.pix8 + b + (base + mg + lane);   // f2 pixel of diagonal a
+    const int all = __reduce_max_sync(FULL, max(ia_lo < ia_hi ? ia_hi + gl - base : 0, ib_lo < ib_hi ? ib_hi + gl - base : 0));
+    const int seg = pass_segment(g, all);
+    int koff = lane / g.nl * seg;
+    W.ka_beg = max(ia_lo + gl - base - koff, 0);
+    W.kb_beg = max(ib_lo + gl - base - koff, 0);
+    W.ka_end = min(ia_hi + gl - base - koff, seg);
+    W.kb_end = min(ib_hi + gl - base - koff, seg);
+    const bool ne_a = ia_lo < ia_hi && W.ka_beg < W.ka_end, ne_b = ib_lo < ib_hi && W.kb_beg < W.kb_end;
+    if (!ne_a) W.ka_beg = W.ka_end = 0;
+    if (!ne_b) W.kb_beg = W.kb_end = 0;
+    if (!ne_a && !ne_b) koff = 0;
+    const double4* __restrict__ A1 = p.pix8 + a + (base - gl + koff);        // f1 pixel of step 0
+    const double4* __restrict__ A2 = p.pix8 + b + (base + mg + gl + koff);   // f2 pixel of diagonal a
     W.acca.zero();
     W.accb.zero();
     W.ra.bx = p.np; W.ra.by = 0; W.ra.k0 = 0; W.ra.lo = 0.0; W.ra.hi = INF; W.ra.sh = INF;
@@ -1186,7 +1228,6 @@ __device__ void item_exact(const CorrParams& p, int64_t t, const SmemHist& h, Re
       W.start(W.rb, exact_e(u, v), exact_s(u, v), W.kb_end, W.kb_beg);
     }
     W.kall = __reduce_max_sync(FULL, max(W.ka_end, W.kb_end));
-    // the loads run at most 34 pixels outside a forest (LYA_MARGIN)
     double4 q1a = A1[0], q2x = A2[0], q2y = A2[1];
     int k = 0;
     for (; k < W.kall; k += 2) {
@@ -1199,7 +1240,7 @@ __device__ void item_exact(const CorrParams& p, int64_t t, const SmemHist& h, Re
       if (((k + 2) & (cap - 1)) == 0)   // bound the length of a run
         W.close(k + 1 >= W.ka_beg && k + 1 < W.ka_end, k + 1 >= W.kb_beg && k + 1 < W.kb_end, k + 2, k + 2);
     }
-    st.evaluated += (unsigned long long)(max(0, W.ka_end - W.ka_beg) + max(0, W.kb_end - W.kb_beg));
+    st.evaluated += (unsigned)(max(0, W.ka_end - W.ka_beg) + max(0, W.kb_end - W.kb_beg));
     W.close(true, true, max(W.ka_end, W.ra.k0), max(W.kb_end, W.rb.k0));
   }
 }
@@ -1246,11 +1287,6 @@ __device__ __forceinline__ void add_compensated(double* hi, double* lo, double v
   if (err != 0.0) atomicAdd(lo, err);
 }
 
-template <int KIND>
-constexpr size_t rec_bytes() {
-  return KIND == LYA_KERNEL_FP32_GUARDED ? sizeof(RecF32) : (KIND == LYA_KERNEL_FP64_DIAGONAL ? sizeof(RecF64) : 0);
-}
-
 // Walk selection of a pair-kernel instance.  The FP32 kernel runs as one
 // instance with the lean walk only (pairs of two lean forests; the others are
 // skipped) followed, when the catalogue has forests the lean walk cannot take,
@@ -1259,7 +1295,12 @@ constexpr size_t rec_bytes() {
 // p.variant names.
 enum { WALK_ANY = 0, WALK_LEAN = 1, WALK_REST = 2 };
 
-// records of a warp's buffer
+// record size and records of a warp's buffer
+template <int KIND, int WALK>
+__host__ __device__ constexpr size_t rec_bytes() {
+  if (KIND == LYA_KERNEL_FP32_GUARDED) return WALK == WALK_LEAN ? sizeof(RecLean) : sizeof(RecF32);
+  return KIND == LYA_KERNEL_FP64_DIAGONAL ? sizeof(RecF64) : 0;
+}
 template <int KIND, int WALK>
 __host__ __device__ constexpr int rec_count() {
   return KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_LEAN ? REC_EXACT : REC;
@@ -1279,18 +1320,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
   unsigned char* bufs = reinterpret_cast<unsigned char*>(h.q + LYA_NQ * nb) + (size_t)nb * sizeof(unsigned long long);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NREC = rec_count<KIND, WALK>();
-  unsigned char* mybuf = bufs + (size_t)warp * NREC * rec_bytes<KIND>();
+  unsigned char* mybuf = bufs + (size_t)warp * NREC * rec_bytes<KIND, WALK>();
   // lean walk: per-warp state and threshold tables after the record buffers; exact walk: its edges
-  unsigned char* tabs = bufs + (size_t)WARPS * NREC * rec_bytes<KIND>();
+  unsigned char* tabs = bufs + (size_t)WARPS * NREC * rec_bytes<KIND, WALK>();
   LeanCtl* myctl = reinterpret_cast<LeanCtl*>(reinterpret_cast<float*>(tabs) + (size_t)warp * lean_ctl_stride(p.np, p.nt));
   double* mytab = reinterpret_cast<double*>(tabs) + (size_t)warp * exact_tab(p.np, p.nt);
   __shared__ unsigned long long s_next;
   __shared__ long long s_seg_end;
   __shared__ int s_slot;
+  __shared__ unsigned long long s_stats[4];   // ST_EVALUATED .. ST_INRANGE
 
+  if (threadIdx.x < 4) s_stats[threadIdx.x] = 0;
   for (int k = threadIdx.x; k < LYA_NQ * nb; k += blockDim.x) h.q[k] = 0.0;
   for (int k = threadIdx.x; k < nb; k += blockDim.x) h.n[k] = 0u;
-  LaneStats st;
   int cnt = 0;   // records pending in this warp's buffer (warp-uniform)
   const int64_t begin = p.cta_begin[blockIdx.x], end = p.cta_begin[blockIdx.x + 1];
   int64_t seg = begin;
@@ -1311,6 +1353,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
     const int64_t seg_end = s_seg_end;
     const int slot = s_slot;
     h.gc = p.counts + (size_t)slot * nb;
+    LaneStats st;
     for (;;) {
       unsigned long long t = 0;
       if (lane == 0) t = atomicAdd(&s_next, 1ull);
@@ -1319,7 +1362,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
       if (KIND == LYA_KERNEL_FP32_GUARDED) {
         if (WALK == WALK_LEAN) {
           if (p.sorted[p.f1[t]] & p.sorted[p.f2[t]] & LYA_LEAN)
-            item_lean(p, (int64_t)t, h, reinterpret_cast<RecF32*>(mybuf), myctl, cnt, st);
+            item_lean(p, (int64_t)t, h, reinterpret_cast<RecLean*>(mybuf), myctl, st);
         } else if (WALK == WALK_REST) {
           if (!(p.sorted[p.f1[t]] & p.sorted[p.f2[t]] & LYA_LEAN))
             item_diag2<TrF32, true>(p, (int64_t)t, h, reinterpret_cast<RecF32*>(mybuf), cnt, st);
@@ -1343,6 +1386,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
     if (KIND == LYA_KERNEL_FP32_GUARDED) drain(reinterpret_cast<RecF32*>(mybuf), cnt, h, nb, st);
     if (KIND == LYA_KERNEL_FP64_DIAGONAL) drain(reinterpret_cast<RecF64*>(mybuf), cnt, h, nb, st);
     cnt = 0;
+    const unsigned stv[4] = {st.evaluated, st.recheck, st.runs, st.inrange};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {   // lane sums can pass 2^32 together: halves apart
+      const unsigned long long v = ((unsigned long long)__reduce_add_sync(FULL, stv[k] >> 16) << 16) +
+                                   __reduce_add_sync(FULL, stv[k] & 0xffffu);
+      if (lane == 0 && v) atomicAdd(&s_stats[k], v);
+    }
     __syncthreads();
     double* gh = p.hist + (size_t)slot * LYA_NQ * 2 * nb;
     for (int k = threadIdx.x; k < LYA_NQ * nb; k += blockDim.x) {
@@ -1365,20 +1415,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
     __syncthreads();
     seg = seg_end;
   }
-  // statistics: one atomic per warp
-  unsigned long long e = st.evaluated, r = st.recheck, u = st.runs, n = st.inrange;
-  for (int o = 16; o > 0; o >>= 1) {
-    e += __shfl_xor_sync(FULL, e, o);
-    r += __shfl_xor_sync(FULL, r, o);
-    u += __shfl_xor_sync(FULL, u, o);
-    n += __shfl_xor_sync(FULL, n, o);
-  }
-  if (lane == 0) {
-    atomicAdd(&p.stats[ST_EVALUATED], e);
-    atomicAdd(&p.stats[ST_RECHECK], r);
-    atomicAdd(&p.stats[ST_RUNS], u);
-    atomicAdd(&p.stats[ST_INRANGE], n);
-  }
+  __syncthreads();
+  if (threadIdx.x < 4 && s_stats[threadIdx.x]) atomicAdd(&p.stats[threadIdx.x], s_stats[threadIdx.x]);
 }
 
 template <int KIND, int WARPS, int WALK>
@@ -1387,7 +1425,7 @@ size_t corr_smem_bytes(const CorrParams& p, int nb) {
   if (KIND == LYA_KERNEL_FP32_GUARDED) tabs = (size_t)WARPS * lean_ctl_stride(p.np, p.nt) * sizeof(float);
   if (KIND == LYA_KERNEL_FP64_DIAGONAL && WALK == WALK_LEAN) tabs = (size_t)WARPS * exact_tab(p.np, p.nt) * sizeof(double);
   return (size_t)nb * (LYA_NQ * sizeof(double) + sizeof(unsigned long long)) +
-         (size_t)WARPS * rec_count<KIND, WALK>() * rec_bytes<KIND>() + tabs;
+         (size_t)WARPS * rec_count<KIND, WALK>() * rec_bytes<KIND, WALK>() + tabs;
 }
 
 template <int KIND, int WARPS, int WALK>

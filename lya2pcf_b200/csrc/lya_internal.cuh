@@ -14,7 +14,7 @@
 #define LYA_MAX_BINS 4096
 #define LYA_WARP 32
 // Zero pixels before the first and after the last forest of the padded pixel
-// arrays: the kernels' software pipelines read up to 34 pixels past either end
+// arrays: the kernels' software pipelines read up to 50 pixels past either end
 // of a forest without bounds checks (the values are never used).
 #define LYA_MARGIN 64
 
