@@ -178,12 +178,13 @@ __global__ void __launch_bounds__(256) k_adjoint(const AdjParams p) {
 //   into a ring of 32 pixels and go to memory 32 pixels at a time.
 // * f2 pixels pass through a ring in shared memory, even and odd pixels apart,
 //   so that the lanes' reads (two pixels apart) are conflict-free.
-// Bound: issue (69% of cycles) with shared-memory wavefronts at 55% and the FP64
-// pipe at 19% (6 operations per pixel pair for both directions; the gather form
+// Bound: issue (72% of cycles) and shared-memory wavefronts (70%); the FP64 pipe
+// is at 25% (6 operations per pixel pair for both directions; the gather form
 // needs 28).  One gradient of 2.80e10 pixel pairs (2,500 forests of 374 pixels):
-// 62.8 ms, the gather form over both directions 99.6 ms; 1.85e9 pairs of
-// 200-pixel forests: 6.0 against 8.6 ms.  24 warps at 80 registers: 20 warps
-// take 70 ms, 28 warps 64.5 ms, 32 warps 67.4 ms.
+// 48.9 ms, the gather form over both directions 99.6 ms; 1.85e9 pairs of
+// 200-pixel forests: 4.56 against 8.6 ms.  24 warps at 80 registers: 20 warps
+// take 50.4 ms, 28 warps 55.3 ms.  Byte offsets in place of indices and 32-bit
+// words for the rt steps: 62.8 -> 48.9 ms.
 constexpr int BAND_WARPS = 24;   // at most (80 registers)
 constexpr int BAND_RING = 128;   // f2 pixels in a warp's ring: 64 in use, 32 ahead, 32 spare
 
@@ -195,16 +196,19 @@ constexpr int BAND_D = 2 * BAND_RING, BAND_OUT = BAND_D + BAND_RING, BAND_EX = B
 __host__ __device__ __forceinline__ int band_table(int np, int nt) { return 2 * (2 * np + 1) * nt; }
 __host__ __device__ __forceinline__ int band_per_warp(int np, int nt) { return BAND_EX + ((2 * np + 1 + nt + 1 + 1) & ~1); }
 extern __shared__ __align__(16) double s_band[];
+// shared memory at a byte offset (rows keep byte offsets: no address arithmetic in the walk)
+__device__ __forceinline__ double band_d(int at) { return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(s_band) + at); }
+__device__ __forceinline__ double2 band_d2(int at) { return *reinterpret_cast<const double2*>(reinterpret_cast<const char*>(s_band) + at); }
 
-// Bin state of a row: the shared-memory offsets ox of the next rp edge and oc of
-// the bin's coefficients, the next rp edge, and the steps kt of its next four rt
-// edges (16 bits each, the nearest lowest).  The row's partners are in range on
+// Bin state of a row: the byte offsets ox of the next rp edge and oc of
+// the bin's coefficients, the next rp edge, and the steps of its next four rt
+// edges (kt, then kt2: 16 bits each, the nearest lowest).  The row's partners are in range on
 // steps kb .. kb + kn - 1.
 struct BandRow {
   double d, w, dw;
   double ex;
   double gdw, gw;
-  unsigned long long kt;
+  unsigned kt, kt2;
   int ox, oc, kb, kn;
 };
 
@@ -218,7 +222,7 @@ __device__ __forceinline__ int edges_passed(int e, int n, double v) {   // entri
 }
 
 __device__ __forceinline__ void band_sums(BandRow& r, int k, const double2& wdw, double& jdw, double& jw) {
-  const double2 c = *reinterpret_cast<const double2*>(&s_band[r.oc]);
+  const double2 c = band_d2(r.oc);
   if ((unsigned)(k - r.kb) < (unsigned)r.kn) {
     r.gdw = __fma_rn(c.x, wdw.y, r.gdw);
     r.gw = __fma_rn(c.y, wdw.x, r.gw);
@@ -231,16 +235,20 @@ __device__ __forceinline__ void band_sums(BandRow& r, int k, const double2& wdw,
 // and one rt edge per step (half of the lanes pass an rp edge at each step of
 // 2 Mpc/h) and at most four rt edges per row, whose steps are known: no branch.
 template <bool SINGLE>
-__device__ __forceinline__ void band_edges(BandRow& r, double d2, int k, int nt2, int es) {
+__device__ __forceinline__ void band_edges(BandRow& r, double d2, int k, int nt16, int es) {
   const double x = __dsub_rn(d2, r.d);
   if (SINGLE) {
-    if (x >= r.ex) { ++r.ox; r.oc += nt2; }
-    r.ex = s_band[r.ox];
-    if (k == (int)(r.kt & 0xffff)) { r.oc += 2; r.kt >>= 16; }
+    if (x >= r.ex) { r.ox += 8; r.oc += nt16; }
+    r.ex = band_d(r.ox);
+    if ((r.kt & 0xffffu) == (unsigned)k) {
+      r.oc += 16;
+      r.kt = __funnelshift_r(r.kt, r.kt2, 16);
+      r.kt2 = r.kt2 >> 16 | 0xffff0000u;
+    }
   } else {
-    while (x >= r.ex) { r.ex = s_band[++r.ox]; r.oc += nt2; }
+    while (x >= r.ex) { r.ox += 8; r.ex = band_d(r.ox); r.oc += nt16; }
     const double s = __dadd_rn(d2, r.d);
-    while (s >= s_band[es + (int)r.kt]) { ++r.kt; r.oc += 2; }   // kt: rt edges passed
+    while (s >= s_band[es + (int)r.kt]) { ++r.kt; r.oc += 16; }   // kt: rt edges passed
   }
 }
 
@@ -248,11 +256,11 @@ __device__ __forceinline__ void band_edges(BandRow& r, double d2, int k, int nt2
 // par (step k), whose sums are jdw, jw.
 template <bool SINGLE>
 __device__ __forceinline__ void band_pair(BandRow& ra, BandRow& rb, int ring, int par, int q, int k, double& jdw,
-                                          double& jw, int nt2, int es) {
-  const double2 wdw = *reinterpret_cast<const double2*>(&s_band[ring + par * BAND_RING + 2 * q]);
-  const double d2 = s_band[ring + BAND_D + par * (BAND_RING / 2) + q];
-  band_edges<SINGLE>(ra, d2, k, nt2, es);
-  band_edges<SINGLE>(rb, d2, k, nt2, es);
+                                          double& jw, int nt16, int es) {
+  const double2 wdw = band_d2(8 * ring + par * 8 * BAND_RING + 16 * q);
+  const double d2 = band_d(8 * ring + 8 * BAND_D + par * 4 * BAND_RING + 8 * q);
+  band_edges<SINGLE>(ra, d2, k, nt16, es);
+  band_edges<SINGLE>(rb, d2, k, nt16, es);
   band_sums(ra, k, wdw, jdw, jw);
   band_sums(rb, k, wdw, jdw, jw);
 }
@@ -265,12 +273,12 @@ struct BandCols {
 // n steps (rounded up to even: a step past the band meets only pairs out of
 // range or outside the forest) from ring position k0.
 template <bool SINGLE>
-__device__ __forceinline__ void band_walk(BandRow& ra, BandRow& rb, BandCols& c, int ring, int k0, int n, int nt2, int es) {
+__device__ __forceinline__ void band_walk(BandRow& ra, BandRow& rb, BandCols& c, int ring, int k0, int n, int nt16, int es) {
   const int lane = threadIdx.x & 31;
   for (int k = 0; k < n; k += 2) {
     const int q = (((k0 + k) >> 1) + lane) & (BAND_RING / 2 - 1);
-    band_pair<SINGLE>(ra, rb, ring, 0, q, k0 + k, c.pdw, c.pw, nt2, es);
-    band_pair<SINGLE>(ra, rb, ring, 1, q, k0 + k + 1, c.qdw, c.qw, nt2, es);
+    band_pair<SINGLE>(ra, rb, ring, 0, q, k0 + k, c.pdw, c.pw, nt16, es);
+    band_pair<SINGLE>(ra, rb, ring, 1, q, k0 + k + 1, c.qdw, c.qw, nt16, es);
     if (lane == 0) {
       *reinterpret_cast<double2*>(&s_band[ring + BAND_OUT + 2 * k]) = make_double2(c.pdw, c.pw);
       *reinterpret_cast<double2*>(&s_band[ring + BAND_OUT + 2 * k + 2]) = make_double2(c.qdw, c.qw);
@@ -289,7 +297,7 @@ __global__ void __launch_bounds__(BAND_WARPS * 32, 1) k_adjoint_band(const AdjPa
     s_band[2 * k] = q < nb ? p.coef[q] : 0.0;
     s_band[2 * k + 1] = q < nb ? p.coef[nb + q] : 0.0;
   }
-  const int nt2 = 2 * nt;
+  const int nt16 = 16 * nt;   // bytes of a coefficient row
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ring = band_table(np, nt) + warp * band_per_warp(np, nt);
   const int ex = ring + BAND_EX, es = ex + 2 * np + 1;
@@ -372,10 +380,10 @@ __global__ void __launch_bounds__(BAND_WARPS * 32, 1) k_adjoint_band(const AdjPa
         const int sx = edges_passed(ex, 2 * np, __dsub_rn(d2, r.d));
         // the rt bin as of the first partner in range
         const int ss = r.kn > 0 ? edges_passed(es, nt, __dadd_rn(D2[r.kb], r.d)) : 0;
-        r.ox = ex + sx;
-        r.oc = sx * nt2 + 2 * ss;
-        r.ex = s_band[r.ox];
-        r.kt = ~0ull;
+        r.ox = 8 * (ex + sx);
+        r.oc = sx * nt16 + 16 * ss;
+        r.ex = s_band[ex + sx];
+        r.kt = r.kt2 = ~0u;
         int at = r.kb;   // the row's partners are at, at + 1, ... end - 1
         const int end = r.kb + r.kn;
         for (int q = 0; at < end; ++q) {   // steps of the rt edges the row passes
@@ -384,7 +392,8 @@ __global__ void __launch_bounds__(BAND_WARPS * 32, 1) k_adjoint_band(const AdjPa
           while (at < hi) { const int k = (at + hi) >> 1; if (__dadd_rn(D2[k], r.d) >= e) hi = k; else at = k + 1; }
           if (at == end) break;
           if (q == 4) { single = false; break; }
-          r.kt = (r.kt & ~(0xffffull << 16 * q)) | (unsigned long long)(at - i - m_lo) << 16 * q;
+          unsigned& word = q < 2 ? r.kt : r.kt2;
+          word = (word & ~(0xffffu << 16 * (q & 1))) | (unsigned)(at - i - m_lo) << 16 * (q & 1);
         }
         if (h) second_ss = ss; else first_ss = ss;
         r.kb -= i + m_lo;
@@ -408,8 +417,8 @@ __global__ void __launch_bounds__(BAND_WARPS * 32, 1) k_adjoint_band(const AdjPa
         stage(k0 + 64);
         __syncwarp();
         const int n = min(32, steps - k0);
-        if (single) band_walk<true>(ra, rb, col, ring, k0, n, nt2, es);
-        else band_walk<false>(ra, rb, col, ring, k0, n, nt2, es);
+        if (single) band_walk<true>(ra, rb, col, ring, k0, n, nt16, es);
+        else band_walk<false>(ra, rb, col, ring, k0, n, nt16, es);
         __syncwarp();
         const int j = j00 + k0 + lane;
         if (lane < ((n + 1) & ~1) && j >= 0 && j < L2) {
