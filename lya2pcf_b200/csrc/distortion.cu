@@ -320,6 +320,19 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
   const int nwm = NW / 4;
   const int mt = warp & 3, ng = warp >> 2;
   const int grp = lane >> 2, kq = lane & 3;
+  // Tiles of a diagonal block, which is symmetric: tile rows r and tile columns
+  // c >= 2r only, dealt to the warps in turn (16 tiles for 50 rp bins, one per
+  // warp, four per SM sub-partition); its columns NS .. NS+3 are the moments.
+  const bool moments_in_tiles = NS + 4 <= 64;
+  int sym_row[CC], sym_col[CC];
+#pragma unroll
+  for (int c = 0; c < CC; ++c) {
+    int x = warp + NW * c, r = 0;
+    const int ncol = (NS + 4 + 7) / 8, nrow = (np + 15) / 16;
+    while (r < nrow && x >= ncol - 2 * r) { x -= ncol - 2 * r; ++r; }
+    sym_row[c] = r < nrow ? r : -1;
+    sym_col[c] = 2 * r + x;
+  }
   unsigned long long n_mma = 0;     // thread 0: MMAs of this CTA
 
   for (;;) {
@@ -599,7 +612,10 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
         }
         __syncthreads();
         const int n = s_cnt;
-        const int nch = (n + CH - 1) / CH;
+        // a diagonal block stages the rows of t only: twice the pixels per chunk
+        const bool wide = diag && moments_in_tiles;
+        const int CB = wide ? 2 * CH : CH, BSET = CB * NPAD;
+        const int nch = (n + CB - 1) / CB;
         // issue the copies of chunk ci into buffer ci & 1 (rows beyond the
         // chunk are zeroed with plain stores).  Columns NS .. NPAD-1 are not
         // copied: they keep older contents, which reach only accumulator
@@ -609,13 +625,13 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
         auto issue = [&](int ci) {
           double* buf = stage + (size_t)(ci & 1) * 4 * SET;
           double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
-          const int c0 = ci * CH, rows = min(CH, n - c0), rows8 = (rows + 7) & ~7;
+          const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
           const int nset = diag ? 2 : 4;           // a diagonal block reads the rows of t only
           const int segs = NS / 2;                 // 16-byte segments of a row
-          // q = (set CH + r) segs + sg over whole chunks; rows r >= rows are skipped
-          for (int q = tid; q < nset * CH * segs; q += DT) {
+          // q = (set CB + r) segs + sg over whole chunks; rows r >= rows are skipped
+          for (int q = tid; q < nset * CB * segs; q += DT) {
             const int sr = segs > 1 ? (int)__umulhi((unsigned)q, seg_magic) : q, sg = q - sr * segs;
-            const int set = sr / CH, r = sr - set * CH;
+            const int set = wide ? sr / (2 * CH) : sr / CH, r = sr - set * CB;
             if (r >= rows) continue;
             const double* colb = (set & 1) ? colL : colS;
             const double* src;
@@ -627,11 +643,11 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               const int bin = set < 2 ? t : u;
               src = colb + (size_t)side * ML * TS * NS + ((size_t)m * TS + (bin - lo)) * NS + 2 * sg;
             }
-            __pipeline_memcpy_async(buf + (size_t)set * SET + (size_t)r * NPAD + 2 * sg, src, 16);
+            __pipeline_memcpy_async(buf + (size_t)set * BSET + (size_t)r * NPAD + 2 * sg, src, 16);
           }
           for (int q = tid; q < nset * (rows8 - rows) * NPAD; q += DT) {
             const int set = q / ((rows8 - rows) * NPAD), rem = q - set * (rows8 - rows) * NPAD;
-            buf[(size_t)set * SET + (size_t)rows * NPAD + rem] = 0.0;
+            buf[(size_t)set * BSET + (size_t)rows * NPAD + rem] = 0.0;
           }
           for (int r = tid - (DT - 32); r >= 0 && r < rows8; r += 32) {   // the last warp
             double ks = 0.0, kl = 0.0, w0 = 0.0, w1 = 0.0;
@@ -642,10 +658,12 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               if (side == 0) { w0 = sw[m]; w1 = sw[m] * sl[m]; }
             }
             kb2[r] = ks;
-            kb2[CH + r] = kl;
-            kb2[2 * CH + r] = w0;
-            kb2[3 * CH + r] = w1;
-            if (diag && NS + 4 <= 64) {   // moment columns of the S and L rows of bin t
+            kb2[CB + r] = kl;
+            if (!wide) {
+              kb2[2 * CH + r] = w0;
+              kb2[3 * CH + r] = w1;
+            }
+            if (diag && moments_in_tiles) {   // moment columns of the S and L rows of bin t
               double dlm = 0.0;
               bool f1r = false;
               if (r < rows) {
@@ -654,7 +672,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
                 dlm = sl[pk & 0xffff];
               }
               double* rs = buf + (size_t)r * NPAD + NS;
-              double* rl = buf + SET + (size_t)r * NPAD + NS;
+              double* rl = buf + BSET + (size_t)r * NPAD + NS;
               rs[0] = f1r ? om2 : 0.0; rs[1] = f1r ? om2 * dlm : 0.0; rs[2] = 0.0; rs[3] = 0.0;
               rl[0] = 0.0; rl[1] = 0.0; rl[2] = f1r ? odl2b : 0.0; rl[3] = f1r ? odl2b * dlm : 0.0;
             }
@@ -673,12 +691,12 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           const double* buf = stage + (size_t)(ci & 1) * 4 * SET;
           const double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
           const double* SA = buf;                      // rows of bin t: S, L (unscaled)
-          const double* LA = buf + SET;
+          const double* LA = buf + BSET;
           const double* SB = diag ? SA : buf + 2 * SET;   // rows of bin u
           const double* LB = diag ? LA : buf + 3 * SET;
-          const int c0 = ci * CH, rows = min(CH, n - c0), rows8 = (rows + 7) & ~7;
+          const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
           if (tid == 0) n_mma += (unsigned long long)((rows + 3) / 4) * ntile * ntile * 2;
-          if (diag && !(NS + 4 <= 64)) {   // moments of bin t from the rows of the f1 pixels
+          if (diag && !moments_in_tiles) {   // moments of bin t from the rows of the f1 pixels
             for (int e = tid; e < 4 * np; e += DT) {
               const int q = e / np, bq = e - q * np;
               const double* src = (q < 2 ? SA : LA) + bq;   // 0: M0, 1: Mi from S; 2: Mj, 3: Mij from L
@@ -689,10 +707,25 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               mom[(q * nt + t) * np + bq] += sacc;
             }
           }
-          {
+          if (diag && moments_in_tiles) {
+#pragma unroll
+            for (int c = 0; c < CC; ++c) {
+              if (sym_row[c] < 0) continue;
+              const int bp0 = 16 * sym_row[c] + grp, bp1 = bp0 + 8, bq = 8 * sym_col[c] + grp;
+              const bool v0 = bp0 < np, v1 = bp1 < np;
+              for (int r0 = 0; r0 < rows8; r0 += 8) {
+                const int ra = (r0 + kq) * NPAD, rb = ra + 4 * NPAD;
+                const double ks0 = kb2[r0 + kq], ks1 = kb2[r0 + kq + 4];
+                const double kl0 = kb2[CB + r0 + kq], kl1 = kb2[CB + r0 + kq + 4];
+                lya_dmma_16x8x8(acc[c], v0 ? SA[ra + bp0] * ks0 : 0.0, v1 ? SA[ra + bp1] * ks0 : 0.0,
+                                v0 ? SA[rb + bp0] * ks1 : 0.0, v1 ? SA[rb + bp1] * ks1 : 0.0, SA[ra + bq], SA[rb + bq]);
+                lya_dmma_16x8x8(acc[c], v0 ? LA[ra + bp0] * kl0 : 0.0, v1 ? LA[ra + bp1] * kl0 : 0.0,
+                                v0 ? LA[rb + bp0] * kl1 : 0.0, v1 ? LA[rb + bp1] * kl1 : 0.0, LA[ra + bq], LA[rb + bq]);
+              }
+            }
+          } else {
             const int bp0 = 16 * mt + grp, bp1 = bp0 + 8;
-            const int arows = (diag && NS + 4 <= 64) ? NS + 4 : np;   // A rows NS..NS+3: the moments
-            const bool v0 = bp0 < arows, v1 = bp1 < arows;
+            const bool v0 = bp0 < np, v1 = bp1 < np;
             for (int r0 = 0; r0 < rows8; r0 += 8) {
               const int ra = (r0 + kq) * NPAD, rb = ra + 4 * NPAD;
               const double ks0 = kb2[r0 + kq], ks1 = kb2[r0 + kq + 4];
@@ -713,51 +746,46 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           }
           __syncthreads();               // buffer ci & 1 is free for chunk ci + 2
         }
-        if (diag && NS + 4 <= 64) {   // accumulator rows NS..NS+3: the moments of bin t
+        if (diag && moments_in_tiles) {   // accumulator columns NS..NS+3: the moments of bin t
 #pragma unroll
-          for (int h2 = 0; h2 < 2; ++h2) {
-            const int q = 16 * mt + grp + 8 * h2 - NS;
-            if (q >= 0 && q < 4) {
+          for (int c = 0; c < CC; ++c) {
 #pragma unroll
-              for (int c = 0; c < CC; ++c) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  const int nt8 = ng + nwm * c, bq = 8 * nt8 + 2 * kq + i;
-                  if (nt8 < ntile && bq < np) mom[(q * nt + t) * np + bq] = acc[c][2 * h2 + i];
-                }
-              }
+            for (int i = 0; i < 4; ++i) {
+              const int bp = 16 * sym_row[c] + grp + 8 * (i >> 1), q = 8 * sym_col[c] + 2 * kq + (i & 1) - NS;
+              if (sym_row[c] >= 0 && bp < np && q >= 0 && q < 4) mom[(q * nt + t) * np + bp] = acc[c][i];
             }
           }
           __syncthreads();
         }
       }
-      // flush: column products (subtracted), rank-4 part, diagonal; warp
-      // (trow, thalf) writes the entries (8 trow + grp, 8c + 2kq + i) of its columns
+      // flush: column products (subtracted), rank-4 part, diagonal.  A diagonal
+      // block from its upper triangle, both halves from one value.
+      const bool sym = diag && moments_in_tiles;
 #pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        const int bp = 16 * mt + grp + 8 * h2;
-        if (bp < np) {
+      for (int c = 0; c < CC; ++c) {
+        const int row = sym ? sym_row[c] : mt, col = sym ? sym_col[c] : ng + nwm * c;
+        if (row < 0 || col >= ntile) continue;
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) {
+          const int bp = 16 * row + grp + 8 * h2;
+          if (bp >= np) continue;
           const double* mtp = mom + (size_t)t * np + bp;   // + q*nt*np
           const double m0a = mtp[0], mia = mtp[nt * np], mja = mtp[2 * nt * np], mija = mtp[3 * nt * np];
 #pragma unroll
-          for (int c = 0; c < CC; ++c) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int nt8 = ng + nwm * c;
-              const int bq = 8 * nt8 + 2 * kq + i;
-              if (nt8 >= ntile || bq >= np) continue;
-              const double* mu = mom + (size_t)u * np + bq;
-              double v = m0a * mu[0] * cA + mja * mu[2 * nt * np] * cB + mia * mu[nt * np] * cC +
-                         mija * mu[3 * nt * np] * cD - acc[c][2 * h2 + i];
-              const int A = bp * nt + t, B = bq * nt + u;
-              if (A == B) {
-                v += m0a;
-                if (m0a != 0.0) atomicAdd(&p.W[A], m0a);
-              }
-              if (v != 0.0) {
-                atomicAdd(&p.D[(size_t)A * nb + B], v);
-                if (t != u) atomicAdd(&p.D[(size_t)B * nb + A], v);
-              }
+          for (int i = 0; i < 2; ++i) {
+            const int bq = 8 * col + 2 * kq + i;
+            if (bq >= np || (sym && bq < bp)) continue;
+            const double* mu = mom + (size_t)u * np + bq;
+            double v = m0a * mu[0] * cA + mja * mu[2 * nt * np] * cB + mia * mu[nt * np] * cC +
+                       mija * mu[3 * nt * np] * cD - acc[c][2 * h2 + i];
+            const int A = bp * nt + t, B = bq * nt + u;
+            if (A == B) {
+              v += m0a;
+              if (m0a != 0.0) atomicAdd(&p.W[A], m0a);
+            }
+            if (v != 0.0) {
+              atomicAdd(&p.D[(size_t)A * nb + B], v);
+              if (t != u || (sym && A != B)) atomicAdd(&p.D[(size_t)B * nb + A], v);
             }
           }
         }
