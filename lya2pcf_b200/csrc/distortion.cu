@@ -28,9 +28,10 @@
 // rows.  Phase 2: the 50x50 (rp x rp) blocks (t, u) of D over the pair's window
 // of rt bins, diagonal blocks first (they complete the moments of bin t, read
 // from the same staged rows: the f1 weights placed in padding columns
-// NS..NS+3 of the staged rows make accumulator rows NS..NS+3 of the diagonal
+// NS..NS+3 of the staged rows make accumulator columns NS..NS+3 of the diagonal
 // block's MMAs the four moments, when NS + 4 <= 64; otherwise a loop over the
-// staged rows).  A block whose rt bins are both spanned by some
+// staged rows; a diagonal block is symmetric, so only the tiles that reach its
+// upper triangle are multiplied).  A block whose rt bins are both spanned by some
 // pixel column gets the column products as a small dense FP64 GEMM on the
 // tensor cores: the rows of the pixels covering t and u are staged in shared
 // memory in chunks of CH pixels, and each warp accumulates 16 x 8 tiles of the
@@ -574,7 +575,8 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
       if (tb >= T0 && tb <= T1) mom[e] = 0.0;
     }
     __syncthreads();
-    const double cA = 1.0 / (om1 * om2), cB = io2 / om1, cC = io1 / om2, cD = io1 * io2;
+    // coefficient of this lane's moment in the rank-4 part (0: M0, 1: Mi, 2: Mj, 3: Mij)
+    const double cq = kq == 0 ? 1.0 / (om1 * om2) : kq == 1 ? io1 / om2 : kq == 2 ? io2 / om1 : io1 * io2;
     // ---- phase 2: blocks (t, u), T0 <= t <= u <= T1, diagonal blocks first.
     // The rows of a chunk of pixels are copied from the column scratch into
     // shared memory asynchronously (16-byte cp.async, no registers), one chunk
@@ -595,6 +597,25 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
       double acc[CC][4];
 #pragma unroll
       for (int c = 0; c < CC; ++c) { acc[c][0] = 0.0; acc[c][1] = 0.0; acc[c][2] = 0.0; acc[c][3] = 0.0; }
+      const bool sym = diag && moments_in_tiles;   // tiles of the upper triangle only
+      // The rank-4 part, subtracted from the tiles as one MMA each with the four
+      // moments as k (lane kq: moment kq; k 4 .. 7 are zero).  Formed per entry in
+      // the flush it read eight moments per pair of entries after the last
+      // barrier: 149.7 against 147.3 ms (72,415 forest pairs).
+      auto rank4 = [&]() {
+        const double* mq = mom + (size_t)kq * nt * np;
+        const double* mt_ = mq + (size_t)t * np;
+        const double* mu_ = mq + (size_t)u * np;
+#pragma unroll
+        for (int c = 0; c < CC; ++c) {
+          const int row = sym ? sym_row[c] : mt, col = sym ? sym_col[c] : ng + nwm * c;
+          if (row < 0 || col >= ntile) continue;
+          const int bp0 = 16 * row + grp, bp1 = bp0 + 8, bq = 8 * col + grp;
+          lya_dmma_16x8x8(acc[c], bp0 < np ? -cq * mt_[bp0] : 0.0, bp1 < np ? -cq * mt_[bp1] : 0.0, 0.0, 0.0,
+                          bq < np ? mu_[bq] : 0.0, 0.0);
+        }
+      };
+      if (!diag) rank4();   // the diagonal blocks have completed the moments
       if (u - t < maxspan) {
         // pixels whose column spans both t and u
         if (tid == 0) s_cnt = 0;
@@ -620,8 +641,8 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
         // chunk are zeroed with plain stores).  Columns NS .. NPAD-1 are not
         // copied: they keep older contents, which reach only accumulator
         // entries that are never flushed (tile columns >= np), except the
-        // moment columns NS .. NS+3 written below for the A rows of a
-        // diagonal block
+        // moment columns NS .. NS+3 written below, tile columns of a diagonal
+        // block
         auto issue = [&](int ci) {
           double* buf = stage + (size_t)(ci & 1) * 4 * SET;
           double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
@@ -758,9 +779,10 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           __syncthreads();
         }
       }
-      // flush: column products (subtracted), rank-4 part, diagonal.  A diagonal
-      // block from its upper triangle, both halves from one value.
-      const bool sym = diag && moments_in_tiles;
+      if (diag) rank4();
+      // flush: the tiles (column products less the rank-4 part) subtracted, the
+      // diagonal added.  A diagonal block from its upper triangle, both halves
+      // from one value.
 #pragma unroll
       for (int c = 0; c < CC; ++c) {
         const int row = sym ? sym_row[c] : mt, col = sym ? sym_col[c] : ng + nwm * c;
@@ -769,23 +791,20 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
         for (int h2 = 0; h2 < 2; ++h2) {
           const int bp = 16 * row + grp + 8 * h2;
           if (bp >= np) continue;
-          const double* mtp = mom + (size_t)t * np + bp;   // + q*nt*np
-          const double m0a = mtp[0], mia = mtp[nt * np], mja = mtp[2 * nt * np], mija = mtp[3 * nt * np];
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const int bq = 8 * col + 2 * kq + i;
             if (bq >= np || (sym && bq < bp)) continue;
-            const double* mu = mom + (size_t)u * np + bq;
-            double v = m0a * mu[0] * cA + mja * mu[2 * nt * np] * cB + mia * mu[nt * np] * cC +
-                       mija * mu[3 * nt * np] * cD - acc[c][2 * h2 + i];
+            double v = -acc[c][2 * h2 + i];
             const int A = bp * nt + t, B = bq * nt + u;
             if (A == B) {
+              const double m0a = mom[(size_t)t * np + bp];
               v += m0a;
               if (m0a != 0.0) atomicAdd(&p.W[A], m0a);
             }
-            if (v != 0.0) {
-              atomicAdd(&p.D[(size_t)A * nb + B], v);
-              if (t != u || (sym && A != B)) atomicAdd(&p.D[(size_t)B * nb + A], v);
+            if (v != 0.0) {   // nb * nb < 2^24
+              atomicAdd(&p.D[A * nb + B], v);
+              if (t != u || (sym && A != B)) atomicAdd(&p.D[B * nb + A], v);
             }
           }
         }
