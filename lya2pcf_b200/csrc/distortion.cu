@@ -309,8 +309,9 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NS = col_stride(np);
-  // q / (NS/2) as a multiply-high: exact for q < 2^16 (the copies of a chunk) and NS > 2
-  const unsigned seg_magic = (unsigned)((0x100000000ull + (unsigned)(NS / 2) - 1) / (unsigned)(NS / 2));
+  // staging: this thread copies 16-byte segment cp_seg of rows cp_row, cp_row + cp_step, ...
+  const int cp_seg = tid % (NS / 2), cp_step = DT / (NS / 2);
+  const int cp_row = tid / (NS / 2) < cp_step ? tid / (NS / 2) : INT_MAX;
   double* colS = p.col + (size_t)blockIdx.x * 2 * 2 * ML * TS * NS;   // [2 sides][ML][TS][NS]
   double* colL = colS + (size_t)2 * ML * TS * NS;
   double* myS = stage + (size_t)warp * 2 * TSB * np;
@@ -648,23 +649,24 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
           const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
           const int nset = diag ? 2 : 4;           // a diagonal block reads the rows of t only
-          const int segs = NS / 2;                 // 16-byte segments of a row
-          // q = (set CB + r) segs + sg over whole chunks; rows r >= rows are skipped
-          for (int q = tid; q < nset * CB * segs; q += DT) {
-            const int sr = segs > 1 ? (int)__umulhi((unsigned)q, seg_magic) : q, sg = q - sr * segs;
-            const int set = wide ? sr / (2 * CH) : sr / CH, r = sr - set * CB;
-            if (r >= rows) continue;
-            const double* colb = (set & 1) ? colL : colS;
-            const double* src;
+          // up to four copies per row offset read; a division by the segments of a
+          // row for every copy takes 147.3 ms instead of 142.3 (72,415 forest pairs)
+          for (int r = cp_row; r < rows; r += cp_step) {
+            int off = 2 * cp_seg;
             if (p.row_offsets) {
-              src = colb + roff[c0 + r] + (set < 2 ? 0 : (u - t) * NS) + 2 * sg;
+              off += roff[c0 + r];
             } else {
               const int pk = plist[c0 + r], side = pk >> 16, m = pk & 0xffff;
-              const int lo = tlo[side * ML + m];
-              const int bin = set < 2 ? t : u;
-              src = colb + (size_t)side * ML * TS * NS + ((size_t)m * TS + (bin - lo)) * NS + 2 * sg;
+              off += ((side * ML + m) * TS + t - tlo[side * ML + m]) * NS;
             }
-            __pipeline_memcpy_async(buf + (size_t)set * BSET + (size_t)r * NPAD + 2 * sg, src, 16);
+            double* dst = buf + r * NPAD + 2 * cp_seg;
+            __pipeline_memcpy_async(dst, colS + off, 16);
+            __pipeline_memcpy_async(dst + BSET, colL + off, 16);
+            if (!diag) {   // rows of u
+              off += (u - t) * NS;
+              __pipeline_memcpy_async(dst + 2 * BSET, colS + off, 16);
+              __pipeline_memcpy_async(dst + 3 * BSET, colL + off, 16);
+            }
           }
           for (int q = tid; q < nset * (rows8 - rows) * NPAD; q += DT) {
             const int set = q / ((rows8 - rows) * NPAD), rem = q - set * (rows8 - rows) * NPAD;
