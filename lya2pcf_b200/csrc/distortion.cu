@@ -99,7 +99,6 @@ struct DistParams {
   unsigned long long* next;// [1] work queue counter
   unsigned long long* mma; // [1] block-product work in m8n8k4 units (8x8 tiles, rows rounded to 4), for the roofline
   int shape;               // launch shape (DIST_SHAPES index); part of the captured graph's key
-  int row_offsets;         // 1: the pixel list carries each pixel's scratch row offset (shared memory allows it)
 };
 
 // Bin of a pixel pair with the reference FP64 formula, as (bp, bt); false when
@@ -294,17 +293,16 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
   double* sd = reinterpret_cast<double*>(smem);          // [2][ML] dc
   double* sw = sd + 2 * ML;                              // [2][ML] w
   double* sl = sw + 2 * ML;                              // [2][ML] dl
-  double* ksc = sl + 2 * ML;                             // [2][ML] column-product weights k_S of a pixel
-  double* klc = ksc + 2 * ML;                            // [2][ML] and k_L
   double* mom = p.moments + (size_t)blockIdx.x * 4 * nt * np;   // [4][nt][np] (CTA-private, L2-resident)
-  double* stage = klc + 2 * ML;                          // 2 x [4][CH][NPAD] staged rows, or the column builders
+  double* stage = sl + 2 * ML;                           // 2 x [4][CH][NPAD] staged rows, or the column builders
   const int stage_len = stage_doubles(CH, NW, np);
   double* kbuf = stage + stage_len;                      // [2][4][CH] per staged row: k_S, k_L, f1 w, f1 w dl
   int* tlo = reinterpret_cast<int*>(kbuf + 8 * CH);      // [2][ML]
   int* span = tlo + 2 * ML;                              // [2][ML]
-  int* plist = span + 2 * ML;                            // [2*ML] packed (side << 16 | pixel)
-  int* roff = plist + 2 * ML;                            // [2*ML] scratch offset of a listed pixel's row t (row_offsets)
-  __shared__ int s_T0, s_T1, s_maxspan, s_cnt;
+  // [2][2*ML] scratch rows of bin t of the pixels of this block and of the next:
+  // (side * ML + pixel) * TS + t - tlo
+  int* rows_of = span + 2 * ML;
+  __shared__ int s_T0, s_T1, s_maxspan, s_cnt[3];
   __shared__ long long s_item;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -355,18 +353,14 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
     const double io2 = p.odl2[b] > 0.0 ? 1.0 / p.odl2[b] : 0.0;
     const bool srt = p.sorted[a] && p.sorted[b], lean = nt <= 64 && (p.sorted[a] & p.sorted[b] & LYA_LEAN);
     const int64_t A0 = p.pstart[a], B0 = p.pstart[b];
-    // pixels, and the weights of their column products: an f1 pixel i enters
-    // with w_i/Om2 (S) and w_i/O2 (L), an f2 pixel j with w_j/Om1 and w_j/O1
     const double kS1 = 1.0 / om2, kS2 = 1.0 / om1;
     for (int k = tid; k < L1; k += DT) {
       const double4 q = p.pix8[A0 + k];
       sd[k] = q.x; sw[k] = q.y; sl[k] = p.dl[A0 + k];
-      ksc[k] = q.y * kS1; klc[k] = q.y * io2;
     }
     for (int k = tid; k < L2; k += DT) {
       const double4 q = p.pix8[B0 + k];
       sd[ML + k] = q.x; sw[ML + k] = q.y; sl[ML + k] = p.dl[B0 + k];
-      ksc[ML + k] = q.y * kS2; klc[ML + k] = q.y * io1;
     }
     if (tid == 0) { s_T0 = INT_MAX; s_T1 = -1; s_maxspan = 0; }
     double* ex = stage;          // [np] exact rp edges (lean pairs; the builders' room is free then)
@@ -571,30 +565,108 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
       __syncthreads();
       continue;
     }
-    for (int e = tid; e < 4 * nt * np; e += DT) {
-      const int tb = (e / np) % nt;
-      if (tb >= T0 && tb <= T1) mom[e] = 0.0;
+    if (!moments_in_tiles) {
+      for (int e = tid; e < 4 * nt * np; e += DT) {
+        const int tb = (e / np) % nt;
+        if (tb >= T0 && tb <= T1) mom[e] = 0.0;
+      }
     }
-    __syncthreads();
     // coefficient of this lane's moment in the rank-4 part (0: M0, 1: Mi, 2: Mj, 3: Mij)
     const double cq = kq == 0 ? 1.0 / (om1 * om2) : kq == 1 ? io1 / om2 : kq == 2 ? io2 / om1 : io1 * io2;
-    // ---- phase 2: blocks (t, u), T0 <= t <= u <= T1, diagonal blocks first.
+    // ---- phase 2: blocks (t, u = t + d) of the window, d = 0 (the diagonal) first.
     // The rows of a chunk of pixels are copied from the column scratch into
     // shared memory asynchronously (16-byte cp.async, no registers), one chunk
     // ahead of the chunk the MMA warps multiply (double buffering); the row
-    // weights k_S, k_L scale the A fragments as the MMA warps read them.
-    const int nT = T1 - T0 + 1;
-    const int nblk = nT + nT * (nT - 1) / 2;
+    // weights k_S, k_L scale the A fragments as the MMA warps read them.  The
+    // chunks of successive blocks form one sequence: the list of the next block's
+    // pixels is built in this block's first chunk, its first chunk is copied
+    // beside this block's last, and there is one barrier per chunk: 142.3 -> 137.0
+    // ms (72,415 forest pairs) against a list, an exposed first chunk and two
+    // barriers a chunk for each block.  Blocks with d >= maxspan have no column
+    // products and come last, without barriers.
+    // Bound: the FP64 MMAs of the blocks (about 35 of the 137 ms at their peak
+    // rate) and the column build, which follow each other in a CTA, issue 46% busy
+    // on the whole; two CTAs of 256 threads per SM, which would overlap them,
+    // take 157.8 ms (chunks of 16, shared loads per MMA).
     const int SET = CH * NPAD;   // doubles of one row set
-    for (int kb = 0; kb < nblk; ++kb) {
-      int t, u;
-      if (kb < nT) { t = u = T0 + kb; }
-      else {   // off-diagonal pairs in row-major order of the upper triangle
-        int r = kb - nT, tt = 0;
-        while (r >= nT - 1 - tt) { r -= nT - 1 - tt; ++tt; }
-        t = T0 + tt; u = t + 1 + r;
+    // pixels whose column spans both t and u = t + d, into list l
+    auto build_list = [&](int t, int d, int l, int* cnt) {
+      for (int side = 0; side < 2; ++side) {
+        const int Lm = side == 0 ? L1 : L2;
+        for (int m = tid; m < Lm; m += DT) {
+          const int lo = tlo[side * ML + m], sp = span[side * ML + m];
+          if (sp > 0 && lo <= t && t + d < lo + sp) {
+            rows_of[l * 2 * ML + atomicAdd(cnt, 1)] = (side * ML + m) * TS + t - lo;   // row u is d further
+          }
+        }
       }
-      const bool diag = t == u;
+    };
+    // a diagonal block stages the rows of t only: twice the pixels per chunk
+    auto chunk_rows = [&](int d) { return d == 0 && moments_in_tiles ? 2 * CH : CH; };
+    // Issues the copies of chunk ci of the block at distance d whose n pixels
+    // are in list l, into buffer gb (rows beyond the chunk are zeroed with plain
+    // stores).  Columns NS .. NPAD-1 are not copied: they keep older contents,
+    // which reach only accumulator entries that are never flushed (tile columns
+    // >= np), except the moment columns NS .. NS+3 written below, tile columns of
+    // a diagonal block.
+    auto issue = [&](int d, int l, int n, int ci, int gb) {
+      const bool diag = d == 0, wide = diag && moments_in_tiles;
+      const int CB = chunk_rows(d), BSET = CB * NPAD;
+      double* buf = stage + (size_t)gb * 4 * SET;
+      double* kb2 = kbuf + (size_t)gb * 4 * CH;
+      const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
+      const int* lr = rows_of + l * 2 * ML + c0;
+      // up to four copies per row offset read; a division by the segments of a
+      // row for every copy takes 147.3 ms instead of 142.3 (72,415 forest pairs)
+      for (int r = cp_row; r < rows; r += cp_step) {
+        int off = lr[r] * NS + 2 * cp_seg;
+        double* dst = buf + r * NPAD + 2 * cp_seg;
+        __pipeline_memcpy_async(dst, colS + off, 16);
+        __pipeline_memcpy_async(dst + BSET, colL + off, 16);
+        if (!diag) {   // rows of u
+          off += d * NS;
+          __pipeline_memcpy_async(dst + 2 * BSET, colS + off, 16);
+          __pipeline_memcpy_async(dst + 3 * BSET, colL + off, 16);
+        }
+      }
+      for (int q = tid; q < (diag ? 2 : 4) * (rows8 - rows) * NPAD; q += DT) {
+        const int set = q / ((rows8 - rows) * NPAD), rem = q - set * (rows8 - rows) * NPAD;
+        buf[(size_t)set * BSET + (size_t)rows * NPAD + rem] = 0.0;
+      }
+      for (int r = tid - (DT - 32); r >= 0 && r < rows8; r += 32) {   // the last warp
+        const bool in = r < rows;
+        const int m = in ? lr[r] / TS : 0, side = m >= ML;   // pixel of both sides' arrays
+        const double wm = sw[m], dlm = sl[m];
+        // weights of the column products: an f1 pixel i enters with w_i/Om2 (S)
+        // and w_i/O2 (L), an f2 pixel j with w_j/Om1 and w_j/O1
+        kb2[r] = in ? wm * (side == 0 ? kS1 : kS2) : 0.0;
+        kb2[CB + r] = in ? wm * (side == 0 ? io2 : io1) : 0.0;
+        const bool f1r = in && side == 0;
+        if (!wide) {
+          kb2[2 * CH + r] = f1r ? wm : 0.0;
+          kb2[3 * CH + r] = f1r ? wm * dlm : 0.0;
+        } else {   // moment columns of the S and L rows of bin t
+          double* rs = buf + (size_t)r * NPAD + NS;
+          double* rl = buf + BSET + (size_t)r * NPAD + NS;
+          rs[0] = f1r ? om2 : 0.0; rs[1] = f1r ? om2 * dlm : 0.0; rs[2] = 0.0; rs[3] = 0.0;
+          rl[0] = 0.0; rl[1] = 0.0; rl[2] = f1r ? odl2b : 0.0; rl[3] = f1r ? odl2b * dlm : 0.0;
+        }
+      }
+      __pipeline_commit();
+    };
+    const int dprod = min(maxspan, T1 - T0 + 1);   // blocks at d < dprod have column products
+    if (tid < 3) s_cnt[tid] = 0;
+    __syncthreads();
+    build_list(T0, 0, 0, &s_cnt[0]);
+    __syncthreads();
+    int gb = 0;                // buffer of the next chunk to multiply
+    int ls = 0;                // counter of the current block's list
+    int l = 0;                 // the current block's list
+    if (s_cnt[0] > 0) issue(0, 0, s_cnt[0], 0, 0);
+    for (int t = T0, d = 0; t + d <= T1;) {
+      const bool diag = d == 0;
+      const int u = t + d;
+      const int tn = t + d < T1 ? t + 1 : T0, dn = t + d < T1 ? d : d + 1;   // the next block
       double acc[CC][4];
 #pragma unroll
       for (int c = 0; c < CC; ++c) { acc[c][0] = 0.0; acc[c][1] = 0.0; acc[c][2] = 0.0; acc[c][3] = 0.0; }
@@ -617,109 +689,34 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
         }
       };
       if (!diag) rank4();   // the diagonal blocks have completed the moments
-      if (u - t < maxspan) {
-        // pixels whose column spans both t and u
-        if (tid == 0) s_cnt = 0;
-        __syncthreads();
-        for (int side = 0; side < 2; ++side) {
-          const int Lm = side == 0 ? L1 : L2;
-          for (int m = tid; m < Lm; m += DT) {
-            const int lo = tlo[side * ML + m], sp = span[side * ML + m];
-            if (sp > 0 && lo <= t && u < lo + sp) {
-              const int x = atomicAdd(&s_cnt, 1);
-              plist[x] = (side << 16) | m;
-              if (p.row_offsets) roff[x] = ((side * ML + m) * TS + t - lo) * NS;   // row u is (u - t) NS further
-            }
-          }
-        }
-        __syncthreads();
-        const int n = s_cnt;
-        // a diagonal block stages the rows of t only: twice the pixels per chunk
-        const bool wide = diag && moments_in_tiles;
-        const int CB = wide ? 2 * CH : CH, BSET = CB * NPAD;
-        const int nch = (n + CB - 1) / CB;
-        // issue the copies of chunk ci into buffer ci & 1 (rows beyond the
-        // chunk are zeroed with plain stores).  Columns NS .. NPAD-1 are not
-        // copied: they keep older contents, which reach only accumulator
-        // entries that are never flushed (tile columns >= np), except the
-        // moment columns NS .. NS+3 written below, tile columns of a diagonal
-        // block
-        auto issue = [&](int ci) {
-          double* buf = stage + (size_t)(ci & 1) * 4 * SET;
-          double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
-          const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
-          const int nset = diag ? 2 : 4;           // a diagonal block reads the rows of t only
-          // up to four copies per row offset read; a division by the segments of a
-          // row for every copy takes 147.3 ms instead of 142.3 (72,415 forest pairs)
-          for (int r = cp_row; r < rows; r += cp_step) {
-            int off = 2 * cp_seg;
-            if (p.row_offsets) {
-              off += roff[c0 + r];
-            } else {
-              const int pk = plist[c0 + r], side = pk >> 16, m = pk & 0xffff;
-              off += ((side * ML + m) * TS + t - tlo[side * ML + m]) * NS;
-            }
-            double* dst = buf + r * NPAD + 2 * cp_seg;
-            __pipeline_memcpy_async(dst, colS + off, 16);
-            __pipeline_memcpy_async(dst + BSET, colL + off, 16);
-            if (!diag) {   // rows of u
-              off += (u - t) * NS;
-              __pipeline_memcpy_async(dst + 2 * BSET, colS + off, 16);
-              __pipeline_memcpy_async(dst + 3 * BSET, colL + off, 16);
-            }
-          }
-          for (int q = tid; q < nset * (rows8 - rows) * NPAD; q += DT) {
-            const int set = q / ((rows8 - rows) * NPAD), rem = q - set * (rows8 - rows) * NPAD;
-            buf[(size_t)set * BSET + (size_t)rows * NPAD + rem] = 0.0;
-          }
-          for (int r = tid - (DT - 32); r >= 0 && r < rows8; r += 32) {   // the last warp
-            double ks = 0.0, kl = 0.0, w0 = 0.0, w1 = 0.0;
-            if (r < rows) {
-              const int pk = plist[c0 + r], side = pk >> 16, m = pk & 0xffff;
-              ks = ksc[side * ML + m];
-              kl = klc[side * ML + m];
-              if (side == 0) { w0 = sw[m]; w1 = sw[m] * sl[m]; }
-            }
-            kb2[r] = ks;
-            kb2[CB + r] = kl;
-            if (!wide) {
-              kb2[2 * CH + r] = w0;
-              kb2[3 * CH + r] = w1;
-            }
-            if (diag && moments_in_tiles) {   // moment columns of the S and L rows of bin t
-              double dlm = 0.0;
-              bool f1r = false;
-              if (r < rows) {
-                const int pk = plist[c0 + r];
-                f1r = (pk >> 16) == 0;
-                dlm = sl[pk & 0xffff];
-              }
-              double* rs = buf + (size_t)r * NPAD + NS;
-              double* rl = buf + BSET + (size_t)r * NPAD + NS;
-              rs[0] = f1r ? om2 : 0.0; rs[1] = f1r ? om2 * dlm : 0.0; rs[2] = 0.0; rs[3] = 0.0;
-              rl[0] = 0.0; rl[1] = 0.0; rl[2] = f1r ? odl2b : 0.0; rl[3] = f1r ? odl2b * dlm : 0.0;
-            }
-          }
-          __pipeline_commit();
-        };
-        if (nch > 0) issue(0);
+      if (d < dprod) {
+        const bool more = dn < dprod && tn + dn <= T1;   // the next block has column products
+        const int ln = l ^ 1, lsn = ls == 2 ? 0 : ls + 1, lsz = lsn == 2 ? 0 : lsn + 1;
+        const int n = s_cnt[ls], CB = chunk_rows(d), BSET = CB * NPAD;
+        const int nch = max((n + CB - 1) / CB, 1);   // an empty list: one step, no rows
         for (int ci = 0; ci < nch; ++ci) {
-          if (ci + 1 < nch) {
-            issue(ci + 1);
-            __pipeline_wait_prior(1);   // this thread's copies of chunk ci have landed
-          } else {
-            __pipeline_wait_prior(0);
+          __pipeline_wait_prior(0);   // this thread's copies of chunk ci have landed
+          __syncthreads();            // everyone's have; the other buffer and the other list are free
+          if (ci == 0) {
+            if (more) build_list(tn, dn, ln, &s_cnt[lsn]);
+            if (tid == 0) s_cnt[lsz] = 0;   // read by everyone in the block before, used in the next
           }
-          __syncthreads();               // everyone's copies of chunk ci have landed
-          const double* buf = stage + (size_t)(ci & 1) * 4 * SET;
-          const double* kb2 = kbuf + (size_t)(ci & 1) * 4 * CH;
+          if (ci + 1 < nch) {
+            issue(d, l, n, ci + 1, gb ^ 1);
+          } else if (more) {
+            if (nch == 1) __syncthreads();   // the next list is complete
+            const int nn = s_cnt[lsn];
+            if (nn > 0) issue(dn, ln, nn, 0, gb ^ 1);
+          }
+          const double* buf = stage + (size_t)gb * 4 * SET;
+          const double* kb2 = kbuf + (size_t)gb * 4 * CH;
           const double* SA = buf;                      // rows of bin t: S, L (unscaled)
           const double* LA = buf + BSET;
           const double* SB = diag ? SA : buf + 2 * SET;   // rows of bin u
           const double* LB = diag ? LA : buf + 3 * SET;
           const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
           if (tid == 0) n_mma += (unsigned long long)((rows + 3) / 4) * ntile * ntile * 2;
-          if (diag && !moments_in_tiles) {   // moments of bin t from the rows of the f1 pixels
+          if (diag && !sym) {   // moments of bin t from the rows of the f1 pixels
             for (int e = tid; e < 4 * np; e += DT) {
               const int q = e / np, bq = e - q * np;
               const double* src = (q < 2 ? SA : LA) + bq;   // 0: M0, 1: Mi from S; 2: Mj, 3: Mij from L
@@ -730,7 +727,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               mom[(q * nt + t) * np + bq] += sacc;
             }
           }
-          if (diag && moments_in_tiles) {
+          if (sym) {
 #pragma unroll
             for (int c = 0; c < CC; ++c) {
               if (sym_row[c] < 0) continue;
@@ -767,9 +764,11 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               }
             }
           }
-          __syncthreads();               // buffer ci & 1 is free for chunk ci + 2
+          gb ^= 1;
         }
-        if (diag && moments_in_tiles) {   // accumulator columns NS..NS+3: the moments of bin t
+        l = ln;
+        ls = lsn;
+        if (sym) {   // accumulator columns NS..NS+3: the moments of bin t
 #pragma unroll
           for (int c = 0; c < CC; ++c) {
 #pragma unroll
@@ -778,8 +777,8 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
               if (sym_row[c] >= 0 && bp < np && q >= 0 && q < 4) mom[(q * nt + t) * np + bp] = acc[c][i];
             }
           }
-          __syncthreads();
         }
+        if (diag) __syncthreads();   // the moments of bin t are complete
       }
       if (diag) rank4();
       // flush: the tiles (column products less the rank-4 part) subtracted, the
@@ -811,6 +810,8 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           }
         }
       }
+      t = tn;
+      d = dn;
     }
     __syncthreads();
   }
@@ -882,6 +883,7 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
   const int shape = ctx->dist_shape;
   const int DT = DIST_SHAPES[shape].dt, CH = DIST_SHAPES[shape].ch, NW = DT / 32;
   const size_t stage_len = (size_t)stage_doubles(CH, NW, np);
+  // the longest forest a shape takes (the layout launched below needs 24 bytes per pixel less)
   const size_t smem = sizeof(double) * (10 * (size_t)max_len + stage_len + 8 * (size_t)CH) +
                       sizeof(int) * (6 * (size_t)max_len);
   if (smem > 227 * 1024)
@@ -921,13 +923,8 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
   p.col = ds.col; p.moments = ds.mom; p.D = ds.D; p.W = ds.W; p.err = ds.err; p.next = ds.err + 1;
   p.mma = ds.err + 3;
   p.shape = shape;
-  size_t smem_run = sizeof(double) * (10 * (size_t)ds.max_len + stage_len + 8 * (size_t)CH) +
-                    sizeof(int) * (6 * (size_t)ds.max_len);
-  // the pixel list's row offsets (one int per listed pixel) when shared memory has room
-  if (smem_run + sizeof(int) * 2 * (size_t)ds.max_len <= 227 * 1024) {
-    smem_run += sizeof(int) * 2 * (size_t)ds.max_len;
-    p.row_offsets = 1;
-  }
+  size_t smem_run = sizeof(double) * (6 * (size_t)ds.max_len + stage_len + 8 * (size_t)CH) +
+                    sizeof(int) * (8 * (size_t)ds.max_len);
   static_assert(sizeof(DistParams) <= sizeof(ds.key), "graph key does not fit");
   cudaError_t e = cudaSuccess;
   if (!ds.graph || memcmp(ds.key, &p, sizeof(p)) != 0) {
