@@ -679,11 +679,11 @@ __device__ void item_diag2(const CorrParams& p, int64_t t, const SmemHist& h, ty
 // an event: the run is closed (record), shifted to the adjacent rp or rt bin
 // when the pair lies inside that bin's interval, otherwise classified again
 // (tables, or the reference FP64 formula inside the guard band).  Sums run over
-// e and s and are scaled to bin units (x = e*cx, y = s*cy) when a run is
-// recorded.  Each lane's first run is classified before the walk, so ragged
-// diagonal starts cost no event; each step takes one warp vote for events (two
-// pairs per lane), and the loop body holds two steps so the pixel registers
-// rotate without copies.
+// e and s and are scaled to bin units (x = e*cx, y = s*cy) when the records are
+// drained.  Each lane's first run is classified before the walk, so ragged
+// diagonal starts cost no event; each step takes one ballot per diagonal, which
+// is both the test for events and the records' positions, and the loop body
+// holds two steps so the pixel registers rotate without copies.
 // Per-warp state of the forest pair being walked, in shared memory (read on
 // the rare paths only, so the walk's registers hold just the runs, the sums and
 // the pixels); the threshold tables follow it: (tlo, thi) of rp bins 0 .. np and
@@ -1022,10 +1022,12 @@ __device__ void item_lean(const CorrParams& p, int64_t t, const SmemHist& h, Rec
 // bin edge by edge.  bx = np: beyond rpmax; a diagonal ends at s >= ty[nt].
 // Two diagonals per lane share the f1 pixel and take one f2 pixel per step: the
 // one-diagonal walk loads two 32-byte pixels per pair and is bound by the L1
-// data pipe (75% busy).  1.50e10 pixel pairs in 37 x 23 bins: 59 ms, the
+// data pipe (75% busy).  1.50e10 pixel pairs in 37 x 23 bins: 49 ms, the
 // one-diagonal walk 102.5 ms; 1.85e9 pairs of 200-pixel forests in 50 x 50 bins:
-// 10.8 against 17.8 ms.  Bound: issue, half of it the runs' events (128
-// registers, 16 warps per SM).
+// 8.25 against 17.8 ms (59 and 10.8 ms before the last pass's split below).
+// Bound: the L1 data pipe again (65-70% busy with two 32-byte pixels per two
+// pairs), issue 45% (128 registers, 16 warps per SM); (dc, w) and (dw, z) in
+// arrays of their own bring the pipe to 54% and the time to 51 ms (spills).
 // Tables of a warp, in shared memory (doubles): ch, sh, tx[np + 2], ty[nt + 2].
 __host__ __device__ __forceinline__ int exact_tab(int np, int nt) { return (2 + np + 2 + nt + 2 + 1) & ~1; }
 
