@@ -893,13 +893,15 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
   // scratch and outputs kept in the context, so later calls (one per healpix
   // pixel in the drop-in driver) allocate nothing and replay the captured graph
   DistScratch& ds = ctx->dist;
-  if (!ds.D || ds.nb != nb || ds.max_len < max_len || ds.grid != grid) {
+  // (binnings of equal nb differ in np, and so in the length of a column's rows)
+  const int stride = col_stride(np);
+  if (!ds.D || ds.nb != nb || ds.max_len < max_len || ds.stride < stride || ds.grid != grid) {
     lya_free(ds.D); lya_free(ds.W); lya_free(ds.col); lya_free(ds.mom); lya_free(ds.err);
     if (ds.graph) { cudaGraphExecDestroy(ds.graph); ds.graph = nullptr; }
     ds = DistScratch{};
     cudaError_t e = lya_alloc(&ds.D, (size_t)nb * nb);
     if (e == cudaSuccess) e = lya_alloc(&ds.W, nb);
-    if (e == cudaSuccess) e = lya_alloc(&ds.col, (size_t)grid * 2 * 2 * max_len * TS * col_stride(np));
+    if (e == cudaSuccess) e = lya_alloc(&ds.col, (size_t)grid * 2 * 2 * max_len * TS * stride);
     if (e == cudaSuccess) e = lya_alloc(&ds.mom, (size_t)grid * 4 * nt * np);
     if (e == cudaSuccess) e = lya_alloc(&ds.err, 4);
     if (e != cudaSuccess) {
@@ -907,7 +909,7 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
       ds = DistScratch{};
       return lya_fail(ctx, LYA_ERR_ALLOC, "lya_dist_run: device allocation failed");
     }
-    ds.nb = nb; ds.max_len = max_len; ds.grid = grid;
+    ds.nb = nb; ds.max_len = max_len; ds.stride = stride; ds.grid = grid;
   }
   cudaStream_t s = ctx->stream;
   const long long n_items = ctx->dist_max_items > 0 ? std::min<long long>(ctx->wq.n_pairs, ctx->dist_max_items)

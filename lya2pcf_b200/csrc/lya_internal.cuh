@@ -115,10 +115,10 @@ struct WorkQueue {
 struct DistScratch {
   double* D = nullptr;                 // [nb][nb]
   double* W = nullptr;                 // [nb]
-  double* col = nullptr;               // column scratch of every CTA
+  double* col = nullptr;               // column scratch of every CTA, rows of `stride` doubles at most
   double* mom = nullptr;               // moment scratch of every CTA
   unsigned long long* err = nullptr;   // [3]: span errors, work counter, item count
-  int nb = 0, max_len = 0, grid = 0;
+  int nb = 0, max_len = 0, stride = 0, grid = 0;
   cudaGraphExec_t graph = nullptr;     // clear + distortion kernel
   alignas(16) unsigned char key[512] = {};   // the kernel parameters it was captured with
 };

@@ -1,0 +1,31 @@
+"""One context used for one call after another: what a call leaves behind (kept
+scratch, captured graphs, CUDA's error state) must not reach the next one."""
+import numpy as np
+import pytest
+
+from lya2pcf_b200 import _native as N
+from lya2pcf_b200.engine import PairEngine
+from oracle import oracle as O
+from test_gpu_edges import all_pairs, ragged
+
+pytestmark = pytest.mark.gpu
+
+
+def _check_distortion(eng, fs, f1, f2, np_, nt):
+    D, W = eng.distortion()
+    Do, Wo = O.distortion(fs, f1, f2, np_=np_, nt=nt)
+    np.testing.assert_allclose(W, Wo, rtol=1e-12, atol=1e-12 * np.abs(Wo).max())
+    assert np.abs(D - Do).max() <= 1e-10 * np.abs(Do).max() and np.abs(Do).max() > 0
+
+
+def test_distortion_binnings_of_equal_size():
+    """np x nt changed at equal np * nt: the rows of the column scratch get
+    longer (and shorter again).  Tolerances of the other distortion tests."""
+    fs = ragged(2.0)
+    f1, f2 = all_pairs(fs)
+    with PairEngine(np_=25, nt=64) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        for np_, nt in ((25, 64), (64, 25), (50, 32), (40, 40)):
+            N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, np_, nt), eng.ctx)
+            _check_distortion(eng, fs, f1, f2, np_, nt)
