@@ -884,9 +884,10 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
   const int DT = DIST_SHAPES[shape].dt, CH = DIST_SHAPES[shape].ch, NW = DT / 32;
   const size_t stage_len = (size_t)stage_doubles(CH, NW, np);
   // the longest forest a shape takes (the layout launched below needs 24 bytes per pixel less)
+  constexpr size_t SMEM_MAX = 227 * 1024;
   const size_t smem = sizeof(double) * (10 * (size_t)max_len + stage_len + 8 * (size_t)CH) +
                       sizeof(int) * (6 * (size_t)max_len);
-  if (smem > 227 * 1024)
+  if (smem > SMEM_MAX)
     return lya_fail(ctx, LYA_ERR_DATA, "lya_dist_run: forests of %d pixels need %zu B of shared memory (shape %d)",
                     max_len, smem, shape);
   const int grid = ctx->num_sms;
@@ -914,19 +915,25 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
   cudaStream_t s = ctx->stream;
   const long long n_items = ctx->dist_max_items > 0 ? std::min<long long>(ctx->wq.n_pairs, ctx->dist_max_items)
                                                     : ctx->wq.n_pairs;
+  // Pixels per forest of the kernel's layout: the scratch's, so that the captured
+  // graph serves any catalogue, unless that is more than this shape holds (a
+  // catalogue of longer forests ran before it, with a shape of smaller chunks).
+  auto layout_bytes = [&](int pixels) {
+    return sizeof(double) * (6 * (size_t)pixels + stage_len + 8 * (size_t)CH) + sizeof(int) * (8 * (size_t)pixels);
+  };
+  const int ml = layout_bytes(ds.max_len) <= SMEM_MAX ? ds.max_len : max_len;
+  const size_t smem_run = layout_bytes(ml);
   DistParams p;
   memset(&p, 0, sizeof(p));   // padding bytes take part in the graph key
   p.pix8 = ctx->cat.pix8; p.dl = ctx->cat.dl; p.pstart = ctx->cat.pstart; p.len = ctx->cat.len;
   p.sorted = ctx->cat.sorted; p.ux = ctx->cat.ux; p.uy = ctx->cat.uy; p.uz = ctx->cat.uz;
   p.omega = ctx->cat.omega; p.odl2 = ctx->cat.odl2; p.f1 = ctx->wq.f1; p.f2 = ctx->wq.f2;
-  p.n_items = reinterpret_cast<const long long*>(ds.err + 2); p.max_len = ds.max_len;
+  p.n_items = reinterpret_cast<const long long*>(ds.err + 2); p.max_len = ml;
   p.binner_rp = (double)np / ctx->rpmax; p.binner_rt = (double)nt / ctx->rtmax;
   p.np = np; p.nt = nt; p.nb = nb; p.cos_variant = ctx->cos_variant; p.npad = npad;
   p.col = ds.col; p.moments = ds.mom; p.D = ds.D; p.W = ds.W; p.err = ds.err; p.next = ds.err + 1;
   p.mma = ds.err + 3;
   p.shape = shape;
-  size_t smem_run = sizeof(double) * (6 * (size_t)ds.max_len + stage_len + 8 * (size_t)CH) +
-                    sizeof(int) * (8 * (size_t)ds.max_len);
   static_assert(sizeof(DistParams) <= sizeof(ds.key), "graph key does not fit");
   cudaError_t e = cudaSuccess;
   if (!ds.graph || memcmp(ds.key, &p, sizeof(p)) != 0) {

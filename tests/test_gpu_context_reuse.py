@@ -3,6 +3,7 @@ scratch, captured graphs, CUDA's error state) must not reach the next one."""
 import numpy as np
 import pytest
 
+from helpers import forestset
 from lya2pcf_b200 import _native as N
 from lya2pcf_b200.engine import PairEngine
 from oracle import oracle as O
@@ -29,3 +30,20 @@ def test_distortion_binnings_of_equal_size():
         for np_, nt in ((25, 64), (64, 25), (50, 32), (40, 40)):
             N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, np_, nt), eng.ctx)
             _check_distortion(eng, fs, f1, f2, np_, nt)
+
+
+def test_distortion_long_forests_then_short():
+    """Forests of 1500 pixels with the launch shape that takes them, then short
+    ones on the same context with the default shape, which does not."""
+    rng = np.random.default_rng(3)
+    line = lambda L, k: dict(ra=0.5 + 0.01 * k, dec=0.1, dc=3600.0 + 0.9 * np.arange(L), w=rng.uniform(0.5, 2.0, L),  # noqa: E731
+                             dw=rng.normal(0, 0.3, L))
+    long = forestset([line(L, k) for k, L in enumerate((1500, 700))])
+    short = forestset([line(L, k) for k, L in enumerate((90, 60, 33))])
+    with PairEngine() as eng:
+        for fs, shape in ((long, 4), (short, 0), (short, 4)):
+            f1, f2 = all_pairs(fs)
+            eng.upload(fs)
+            eng.set_pairs(f1, f2)
+            N.check(eng.lib.lya_dist_config(eng.ctx, shape, 0), eng.ctx)
+            _check_distortion(eng, fs, f1, f2, 50, 50)
