@@ -97,7 +97,9 @@ struct DistParams {
   double* W;               // [nb]
   unsigned long long* err; // [1] pixels whose column spans more than TS rt bins
   unsigned long long* next;// [1] work queue counter
-  unsigned long long* mma; // [1] block-product work in m8n8k4 units (8x8 tiles, rows rounded to 4), for the roofline
+  // [1] block-product work in m8n8k4 units, for the roofline: 8x8 tiles of a block (of a diagonal block, the
+  // tiles that are multiplied for its upper triangle and the moments), pixels rounded to 4
+  unsigned long long* mma;
   int shape;               // launch shape (DIST_SHAPES index); part of the captured graph's key
 };
 
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
   // c >= 2r only, dealt to the warps in turn (16 tiles for 50 rp bins, one per
   // warp, four per SM sub-partition); its columns NS .. NS+3 are the moments.
   const bool moments_in_tiles = NS + 4 <= 64;
-  int sym_row[CC], sym_col[CC];
+  int sym_row[CC], sym_col[CC], sym_tiles = 0;   // sym_tiles: as 8x8 tiles
 #pragma unroll
   for (int c = 0; c < CC; ++c) {
     int x = warp + NW * c, r = 0;
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
     sym_row[c] = r < nrow ? r : -1;
     sym_col[c] = 2 * r + x;
   }
+  for (int r = 0; 16 * r < np; ++r) sym_tiles += ((NS + 4 + 7) / 8 - 2 * r) * min(2, ntile - 2 * r);
   unsigned long long n_mma = 0;     // thread 0: MMAs of this CTA
 
   for (;;) {
@@ -715,7 +718,7 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
           const double* SB = diag ? SA : buf + 2 * SET;   // rows of bin u
           const double* LB = diag ? LA : buf + 3 * SET;
           const int c0 = ci * CB, rows = min(CB, n - c0), rows8 = (rows + 7) & ~7;
-          if (tid == 0) n_mma += (unsigned long long)((rows + 3) / 4) * ntile * ntile * 2;
+          if (tid == 0) n_mma += (unsigned long long)((rows + 3) / 4) * (sym ? sym_tiles : ntile * ntile) * 2;
           if (diag && !sym) {   // moments of bin t from the rows of the f1 pixels
             for (int e = tid; e < 4 * np; e += DT) {
               const int q = e / np, bq = e - q * np;

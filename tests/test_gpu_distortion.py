@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import edge_cases as E
+from helpers import forestset
 from lya2pcf_b200 import _native as N
 from lya2pcf_b200 import synthetic
 from lya2pcf_b200.dropin_path import ensure_on_path
@@ -189,3 +190,40 @@ def test_every_launch_shape_and_the_item_limit():
         assert 0 <= tune['best'] < len(PairEngine.DIST_SHAPES)
         D, W = eng.distortion()
         _check(D, W, Do, Wo)
+
+
+@pytest.mark.parametrize('np_', [50, 37, 64])
+def test_mma_flops_count_the_products_made(np_):
+    """dist_mma_flops of one forest pair from the columns' spans: off-diagonal
+    blocks multiply every 8x8 tile, diagonal blocks those of the 16-row tiles
+    that reach the upper triangle (with the columns of the moments), except
+    where 64 rp bins leave the moments no column."""
+    nt, L, sep = 50, 150, 0.02
+    rng = np.random.default_rng(11)
+    dc = 3600.0 + 2.0 * np.arange(L)
+    fs = forestset([dict(ra=0.5 + sep * k, dec=0.0, dc=dc + 0.3 * k, w=rng.uniform(0.5, 2.0, L), dw=rng.normal(0, 0.3, L))
+                    for k in range(2)])
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(np.array([0]), np.array([1]))
+        eng.distortion()
+        flops = eng.stats()['dist_mma_flops']
+    ch, sh = np.cos(sep / 2), np.sin(sep / 2)
+    d1, d2 = fs.forest(0)['dc'][:, None], fs.forest(1)['dc'][None]
+    bp, bt = np.floor(abs(d1 - d2) * ch * np_ / 200), np.floor((d1 + d2) * sh * nt / 200)
+    inside = (bp < np_) & (bt < nt)
+    lo = np.concatenate([np.where(inside, bt, np.inf).min(axis) for axis in (1, 0)])
+    hi = np.concatenate([np.where(inside, bt, -1).max(axis) for axis in (1, 0)])
+    span = np.where(hi >= lo, hi - lo + 1, 0)
+    ntile, stride = -(-np_ // 8), np_ + np_ % 2
+    moments = stride + 4 <= 64
+    sym = sum((-(-(stride + 4) // 8) - 2 * r) * min(2, ntile - 2 * r) for r in range(-(-np_ // 16)))
+    T0, T1 = int(lo[span > 0].min()), int(hi.max())
+    assert span.max() > 1 and T1 > T0
+    units = 0
+    for d in range(int(min(span.max(), T1 - T0 + 1))):
+        for t in range(T0, T1 - d + 1):
+            n = int(((lo <= t) & (t + d <= hi) & (span > 0)).sum())
+            chunk, tiles = (64, sym) if d == 0 and moments else (32, ntile ** 2)
+            units += 2 * tiles * sum(-(-min(chunk, n - c) // 4) for c in range(0, n, chunk))
+    assert flops == units * 2 * 8 * 8 * 4
