@@ -711,13 +711,17 @@ struct LeanRun {
   float lo, hi, sh;
 };
 
-// A run's record: bin and length packed (4096 bins, runs of at most 1024 pairs),
-// the sums of w12 e and w12 s not yet scaled to bin units.
+// A run's record: bin and length packed (runs of at most 1024 pairs), the sums
+// of w12 e and w12 s not yet scaled to bin units.  A run beyond rpmax is written
+// with length 0 and the bin that its state (np, by) gives, up to nb + nt: such
+// an index must not reach the length's bits, which lean_records_fit checks
+// before a launch (length and bin chosen apart per record costs the walk 2%).
 struct __align__(8) RecLean {
-  unsigned key;   // n << 12 | bin
+  unsigned key;   // n << LEAN_BIN_BITS | bin
   float aw, adw, ae, as, az;
 };
-static_assert(LYA_MAX_BINS <= 4096, "a record's bin has 12 bits");
+constexpr int LEAN_BIN_BITS = 12;
+static bool lean_records_fit(int nb, int nt) { return nb + nt < 1 << LEAN_BIN_BITS; }
 
 struct LeanAcc {
   float aw, adw, ae, as, az;
@@ -813,7 +817,7 @@ __device__ __forceinline__ void lean_drain(const RecLean* buf, int cnt, const Le
   const float cxf = c->cxf, cyf = c->cyf;
   for (int k = threadIdx.x & 31; k < cnt; k += 32) {
     const RecLean r = buf[k];
-    const unsigned bin = r.key & 4095u, n = r.key >> 12;
+    const unsigned bin = r.key & ((1u << LEAN_BIN_BITS) - 1u), n = r.key >> LEAN_BIN_BITS;
     if (n == 0) continue;
     if (bin >= (unsigned)nb) {   // never written by a correct walk: report, skip
       atomicOr(h.err, 1ull);
@@ -846,7 +850,7 @@ struct LeanWalk {
   __device__ __forceinline__ void record(bool w, const LeanRun& r, const LeanAcc& acc, int k, int pos) {
     if (w) {
       RecLean rec;
-      rec.key = (r.bx < p.np ? (unsigned)(k - r.k0) << 12 : 0u) | (unsigned)(r.bx * p.nt + r.by);
+      rec.key = (r.bx < p.np ? (unsigned)(k - r.k0) << LEAN_BIN_BITS : 0u) | (unsigned)(r.bx * p.nt + r.by);
       rec.aw = acc.aw; rec.adw = acc.adw; rec.ae = acc.ae; rec.as = acc.as; rec.az = acc.az;
       buf[pos] = rec;
     }
@@ -1670,6 +1674,9 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
     }
     if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_corr_run: %s", cudaGetErrorString(e));
   }
+  // (the shared memory ends well before: 3,150 bins)
+  if (kind == LYA_KERNEL_FP32_GUARDED && !lean_records_fit(nb, ctx->nt))
+    return lya_fail(ctx, LYA_ERR_ARG, "lya_corr_run: %d x %d bins exceed the FP32 walk's records", ctx->np, ctx->nt);
   static_assert(sizeof(RunGraphKey) <= sizeof(ctx->run_graph_key), "graph key does not fit the context");
   if (!ctx->run_graph || memcmp(&ctx->run_graph_key, &key, sizeof(key)) != 0) {
     if (ctx->run_graph) { cudaGraphExecDestroy(ctx->run_graph); ctx->run_graph = nullptr; }
