@@ -76,11 +76,25 @@ struct CorrParams {
   unsigned long long* stats;    // [ST_N]
 };
 
-// Statistics of a lane within one owner slot's segment, added to the CTA's
-// 64-bit sums at its end (64-bit lane sums would hold eight registers through
-// the walks).
+// Statistics of a lane, added to the CTA's 64-bit sums at the end of an owner
+// slot's segment, and after any forest pair that brought one to 2^30 (64-bit lane
+// sums would hold eight registers through the walks).  A pair adds at most
+// L1 L2 / 32 to a lane's largest: below 2^31 for forests of up to 180,000 pixels.
 struct LaneStats {
   unsigned evaluated = 0, recheck = 0, runs = 0, inrange = 0;
+
+  __device__ __forceinline__ bool large() const { return (evaluated | inrange) >> 30 != 0; }
+  // all lanes of the warp
+  __device__ __forceinline__ void add_to(unsigned long long* sums) {
+    const unsigned v[4] = {evaluated, recheck, runs, inrange};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {   // lane sums can pass 2^32 together: halves apart
+      const unsigned long long t = ((unsigned long long)__reduce_add_sync(0xffffffffu, v[k] >> 16) << 16) +
+                                   __reduce_add_sync(0xffffffffu, v[k] & 0xffffu);
+      if ((threadIdx.x & 31) == 0 && t) atomicAdd(&sums[k], t);
+    }
+    evaluated = recheck = runs = inrange = 0;
+  }
 };
 
 // Shared-memory histogram of the slot being accumulated.
@@ -1388,17 +1402,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_corr(const CorrParams p) {
         else item_diag<TrF64, false>(p, (int64_t)t, h, reinterpret_cast<RecF64*>(mybuf), cnt, st);
       }
       else item_plain(p, (int64_t)t, h, st);
+      if (__any_sync(FULL, st.large())) st.add_to(s_stats);
     }
     if (KIND == LYA_KERNEL_FP32_GUARDED) drain(reinterpret_cast<RecF32*>(mybuf), cnt, h, nb, st);
     if (KIND == LYA_KERNEL_FP64_DIAGONAL) drain(reinterpret_cast<RecF64*>(mybuf), cnt, h, nb, st);
     cnt = 0;
-    const unsigned stv[4] = {st.evaluated, st.recheck, st.runs, st.inrange};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {   // lane sums can pass 2^32 together: halves apart
-      const unsigned long long v = ((unsigned long long)__reduce_add_sync(FULL, stv[k] >> 16) << 16) +
-                                   __reduce_add_sync(FULL, stv[k] & 0xffffu);
-      if (lane == 0 && v) atomicAdd(&s_stats[k], v);
-    }
+    st.add_to(s_stats);
     __syncthreads();
     double* gh = p.hist + (size_t)slot * LYA_NQ * 2 * nb;
     for (int k = threadIdx.x; k < LYA_NQ * nb; k += blockDim.x) {
