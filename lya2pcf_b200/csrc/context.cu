@@ -57,6 +57,9 @@ int lya_fail(lya_ctx* ctx, int code, const char* fmt, ...) {
   va_end(ap);
   g_thread_err = buf;
   if (ctx) ctx->err = buf;
+  // A refused call (shared memory, an allocation) leaves its error in the runtime,
+  // where the next launch's check would find it and fail a sound call.
+  (void)cudaGetLastError();
   return code;
 }
 

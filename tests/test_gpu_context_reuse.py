@@ -47,3 +47,33 @@ def test_distortion_long_forests_then_short():
             eng.set_pairs(f1, f2)
             N.check(eng.lib.lya_dist_config(eng.ctx, shape, 0), eng.ctx)
             _check_distortion(eng, fs, f1, f2, 50, 50)
+
+
+def test_a_refused_run_leaves_no_error_behind():
+    """A binning beyond the shared memory is refused; the next calls, on this
+    context and on a new one, are not."""
+    fs = ragged(2.0)
+    f1, f2 = all_pairs(fs)
+    slot_start = np.searchsorted(fs.pix[f1], np.arange(fs.pix[-1] + 2))
+    expect = O.corr(fs, f1, f2, slot_start)[1]
+
+    def counts(eng):
+        eng.run(kernel=N.KERNEL_FP64_DIAGONAL)
+        return eng.histograms()[1]
+
+    with PairEngine(np_=64, nt=64) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        for kernel in (N.KERNEL_FP32_GUARDED, N.KERNEL_FP64_DIAGONAL):
+            with pytest.raises(N.LyaError):
+                eng.run(kernel=kernel)
+            with PairEngine() as other:
+                other.upload(fs)
+                other.set_pairs(f1, f2)
+                assert np.array_equal(counts(other), expect)
+            with pytest.raises(N.LyaError):
+                eng.run(kernel=kernel)
+            N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, 50, 50), eng.ctx)
+            eng.nb = 2500
+            assert np.array_equal(counts(eng), expect)
+            N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, 64, 64), eng.ctx)
