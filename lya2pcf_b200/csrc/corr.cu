@@ -1459,13 +1459,16 @@ cudaError_t launch_corr(const CorrParams& p, int nctas, int nb, cudaStream_t s) 
 // instance for the pairs it skips when the catalogue has forests it cannot take.
 static bool fp32_lean_walk(int variant) { return variant == 0 || variant == 3; }
 
-// The FP64 kernel's default walk is the exact walk (and the one-diagonal walk
-// for the pairs it skips) when its records and edge tables fit the shared memory
-// beside the histogram: every binning the one-diagonal walk fits with np + nt up
-// to 180, and 2,500 bins with np + nt up to 290.
+// The FP64 kernel's default walk is the exact walk, with the one-diagonal walk
+// for the pairs it skips, when both fit the shared memory beside the histogram:
+// the exact walk its edge tables and 80 records per warp, the other 128 records.
+// Whether a binning is taken does then not depend on the catalogue: the walks
+// share the limit of 2,773 bins, up to which the edge tables fit for np + nt up
+// to 280 (2,500 bins: up to 380).
 static bool fp64_exact_walk(const CorrParams& p, int nb) {
-  return p.variant == 0 &&
-         corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, nb) <= 226 * 1024;
+  constexpr size_t ROOM = 226 * 1024;
+  return p.variant == 0 && corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, nb) <= ROOM &&
+         corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, nb) <= ROOM;
 }
 
 // ------------------------------------------------------------------ CTA ranges

@@ -113,3 +113,25 @@ def test_fp64_walk_edges(np_, nt, step, unsorted):
             for q in (N.Q_W, N.Q_DW, N.Q_RP, N.Q_RT, N.Q_Z):
                 scale = hist[:, O.Q_DWABS if q == N.Q_DW else q]
                 assert np.all(np.abs(h[:, q] - hist[:, q]) <= 1e-12 * scale), q
+
+
+@pytest.mark.parametrize('unsorted', [False, True])
+@pytest.mark.parametrize('np_,nt,fits', [(53, 52, True), (47, 59, True), (53, 53, False), (64, 44, False)])
+def test_fp64_binnings_taken(np_, nt, fits, unsorted):
+    """Binnings around the shared memory's limit are taken or refused whatever
+    the forests are; a refused one leaves the context usable."""
+    fs = ragged(2.0, unsorted)
+    f1, f2 = all_pairs(fs)
+    slot_start = np.searchsorted(fs.pix[f1], np.arange(fs.pix[-1] + 2))
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        if not fits:
+            with pytest.raises(N.LyaError):
+                eng.run(kernel=N.KERNEL_FP64_DIAGONAL)
+            np_ = nt = 50
+            N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, np_, nt), eng.ctx)
+            eng.nb = np_ * nt
+        eng.run(kernel=N.KERNEL_FP64_DIAGONAL)
+        _, c = eng.histograms()
+    assert np.array_equal(c, O.corr(fs, f1, f2, slot_start, np_=np_, nt=nt)[1])
