@@ -542,9 +542,9 @@ int lya_adjoint_launch(lya_ctx* ctx, const double* g, double* grad_dw, double* g
     } else {
       k_unpad<<<blocks, 128, 0, s>>>(n, d_start, ctx->cat.pstart, gdw, out);
       ctx->launches++;
-      lya_touch_pages(grad_dw, sizeof(double) * npix);   // beside the kernels
-      lya_touch_pages(grad_w, sizeof(double) * npix);
-      if (grad_dw) e = cudaMemcpyAsync(grad_dw, out, sizeof(double) * npix, cudaMemcpyDeviceToHost, s);
+      e = lya_touch_pages(grad_dw, sizeof(double) * npix);   // beside the kernels
+      if (e == cudaSuccess) e = lya_touch_pages(grad_w, sizeof(double) * npix);
+      if (e == cudaSuccess && grad_dw) e = cudaMemcpyAsync(grad_dw, out, sizeof(double) * npix, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       k_unpad<<<blocks, 128, 0, s>>>(n, d_start, ctx->cat.pstart, gw, out);
       ctx->launches++;

@@ -63,9 +63,14 @@ int lya_fail(lya_ctx* ctx, int code, const char* fmt, ...) {
   return code;
 }
 
-void lya_touch_pages(void* p, size_t bytes) {
+cudaError_t lya_touch_pages(void* p, size_t bytes) {
   constexpr size_t PAGE = 4096, SHARE = size_t(1) << 20;
-  if (!p || bytes < 2 * SHARE) return;
+  if (!p) return cudaSuccess;
+  cudaPointerAttributes at;
+  const cudaError_t e = cudaPointerGetAttributes(&at, p);
+  if (e != cudaSuccess) return e;
+  if (at.type == cudaMemoryTypeDevice) return cudaErrorInvalidValue;
+  if (at.type != cudaMemoryTypeUnregistered || bytes < 2 * SHARE) return cudaSuccess;
   auto touch = [p, bytes](size_t from, size_t to) {
     for (size_t k = from; k < to && k < bytes; k += PAGE) __atomic_fetch_or(static_cast<char*>(p) + k, 0, __ATOMIC_RELAXED);
   };
@@ -84,6 +89,7 @@ void lya_touch_pages(void* p, size_t bytes) {
   touch(0, share);
   if (started + 1 < n) touch((started + 1) * share, bytes);
   for (unsigned k = 0; k < started; ++k) helpers[k].join();
+  return cudaSuccess;
 }
 
 void lya_free_catalog(DevCatalog& c) {
@@ -661,14 +667,14 @@ extern "C" int lya_corr_get(lya_ctx* ctx, int32_t slot_first, int32_t n, double*
     k_combine<<<blocks, 256, 0, ctx->stream>>>(n, nb, src, tmp);
     ctx->launches++;
     e = cudaGetLastError();
-    lya_touch_pages(hist, sizeof(double) * (size_t)n * LYA_NQ * nb);
+    if (e == cudaSuccess) e = lya_touch_pages(hist, sizeof(double) * (size_t)n * LYA_NQ * nb);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(hist, tmp, sizeof(double) * (size_t)n * LYA_NQ * nb, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_corr_get: %s", cudaGetErrorString(e));
   }
   if (counts) {
-    lya_touch_pages(counts, sizeof(unsigned long long) * (size_t)n * nb);
+    LYA_CHECK_CUDA(ctx, lya_touch_pages(counts, sizeof(unsigned long long) * (size_t)n * nb));
     LYA_CHECK_CUDA(ctx, cudaMemcpyAsync(counts, ctx->counts + (size_t)slot_first * nb,
                                         sizeof(unsigned long long) * (size_t)n * nb, cudaMemcpyDeviceToHost,
                                         ctx->stream));

@@ -233,7 +233,7 @@ extern "C" int lya_covariance(lya_ctx* ctx, int64_t n_rows, const double* xi, co
   }
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, s);
   unsigned long long nzero = 0;
-  lya_touch_pages(cov, sizeof(double) * (size_t)nb * nb);   // beside the kernels
+  if (e == cudaSuccess) e = lya_touch_pages(cov, sizeof(double) * (size_t)nb * nb);   // beside the kernels
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nzero, d_zero, sizeof(nzero), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && mean) e = cudaMemcpyAsync(mean, d_mean, sizeof(double) * nb, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && cov)
@@ -288,7 +288,7 @@ extern "C" int lya_covariance_smooth(lya_ctx* ctx, const double* cov, double* co
       ctx->launches += 2;
       e = cudaGetLastError();
     }
-    lya_touch_pages(cov_smooth, sizeof(double) * (size_t)nb * nb);   // beside the kernels
+    if (e == cudaSuccess) e = lya_touch_pages(cov_smooth, sizeof(double) * (size_t)nb * nb);   // beside the kernels
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(cov_smooth, d_out, sizeof(double) * (size_t)nb * nb, cudaMemcpyDeviceToHost, s);
   } else if (e == cudaSuccess) {

@@ -971,7 +971,7 @@ extern "C" int lya_dist_run(lya_ctx* ctx, double* D, double* W) {
     e = cudaEventRecord(ctx->ev1, s);
   }
   unsigned long long nerr = 0, nmma = 0;
-  lya_touch_pages(D, sizeof(double) * (size_t)nb * nb);   // beside the kernel
+  if (e == cudaSuccess) e = lya_touch_pages(D, sizeof(double) * (size_t)nb * nb);   // beside the kernel
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nerr, ds.err, sizeof(nerr), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nmma, ds.err + 3, sizeof(nmma), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && D) e = cudaMemcpyAsync(D, ds.D, sizeof(double) * (size_t)nb * nb, cudaMemcpyDeviceToHost, s);

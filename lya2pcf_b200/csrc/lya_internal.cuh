@@ -252,8 +252,10 @@ inline cudaError_t lya_alloc(T** p, size_t count) {
 // written takes a fault per page inside the driver's own single-threaded copy:
 // 50 MB took 22.8 ms in 4 KB pages where the copy itself takes 2.5 ms; 8 threads
 // back them in 2.6 ms, and callers let that run beside the kernels.  Buffers
-// below 2 MB are left alone (a thread start costs as much as their faults).
-void lya_touch_pages(void* p, size_t bytes);
+// below 2 MB are left alone (a thread start costs as much as their faults), as
+// are those that CUDA knows (pinned, managed).  Device memory given as a host
+// output is an error, found before anything touches it.  A NULL buffer is none.
+cudaError_t lya_touch_pages(void* p, size_t bytes);
 
 template <typename T>
 inline void lya_free(T*& p) {

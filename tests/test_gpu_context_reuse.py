@@ -1,5 +1,7 @@
 """One context used for one call after another: what a call leaves behind (kept
 scratch, captured graphs, CUDA's error state) must not reach the next one."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -77,3 +79,28 @@ def test_a_refused_run_leaves_no_error_behind():
             eng.nb = 2500
             assert np.array_equal(counts(eng), expect)
             N.check(eng.lib.lya_set_bins(eng.ctx, 200.0, 200.0, 64, 64), eng.ctx)
+
+
+@pytest.mark.parametrize('nb_side', [50, 10])
+def test_device_memory_as_a_host_output_is_refused(nb_side):
+    """Device pointers where the library writes host results (of more and of
+    less than 2 MB): an error status, and the context stays usable."""
+    import torch
+    nb = nb_side ** 2
+    rng = np.random.default_rng(2)
+    xi, w = rng.normal(size=(6, nb)), rng.uniform(1.0, 2.0, (6, nb))
+    dev = torch.zeros(nb * nb, dtype=torch.float64, device='cuda')
+    with PairEngine(np_=nb_side, nt=nb_side) as eng:
+        mean, out, smooth = np.zeros(nb), np.zeros((nb, nb)), np.zeros((nb, nb))
+        cov = lambda ptr: eng.lib.lya_covariance(eng.ctx, 6, N.ptr(xi), N.ptr(w), N.ptr(mean), ptr)  # noqa: E731
+        N.check(cov(N.ptr(out)), eng.ctx)
+        first = out.copy()
+        assert cov(C.c_void_p(dev.data_ptr())) == 2
+        out[:] = 0
+        N.check(cov(N.ptr(out)), eng.ctx)
+        np.testing.assert_array_equal(out, first)
+        sm = C.c_int32(0)
+        assert eng.lib.lya_covariance_smooth(eng.ctx, None, C.c_void_p(dev.data_ptr()), C.byref(sm)) == 2
+        N.check(eng.lib.lya_covariance_smooth(eng.ctx, None, N.ptr(smooth), C.byref(sm)), eng.ctx)
+        assert sm.value == 1 and np.isfinite(smooth).all()
+    assert float(dev.abs().max()) == 0.0
