@@ -135,3 +135,25 @@ def test_fp64_binnings_taken(np_, nt, fits, unsorted):
         eng.run(kernel=N.KERNEL_FP64_DIAGONAL)
         _, c = eng.histograms()
     assert np.array_equal(c, O.corr(fs, f1, f2, slot_start, np_=np_, nt=nt)[1])
+
+
+@pytest.mark.parametrize('np_,nt,where', [(50, 72, 'lean'), (37, 100, 'lean'), (37, 23, 'negative'), (50, 50, 'negative'),
+                                          (64, 60, 'far'), (31, 50, 'far')])
+def test_distortion_sorted_forests_of_the_general_builder(np_, nt, where):
+    """Sorted forests whose columns are not built from edges: more than 64 rt
+    bins, or distances that are negative or above 1e6.  Same tolerances."""
+    fs = ragged(2.0)
+    if where == 'negative':
+        for f in range(fs.n):
+            a, b = int(fs.start[f]), int(fs.start[f + 1])
+            fs.dc[a:b] -= fs.dc[a] + 50.0
+    elif where == 'far':
+        fs.dc += 1e6
+    f1, f2 = all_pairs(fs)
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        D, W = eng.distortion()
+    Do, Wo = O.distortion(fs, f1, f2, np_=np_, nt=nt)
+    np.testing.assert_allclose(W, Wo, rtol=1e-12, atol=1e-12 * np.abs(Wo).max())
+    assert np.abs(D - Do).max() <= 1e-10 * np.abs(Do).max() and np.abs(Do).max() > 0
