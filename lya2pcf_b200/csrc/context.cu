@@ -206,7 +206,7 @@ extern "C" int lya_ctx_create(int device, lya_ctx** out) {
     if ((e = cudaEventCreate(&ctx->ev3)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
     if ((e = cudaEventCreate(&ctx->tev0)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
     if ((e = cudaEventCreate(&ctx->tev1)) != cudaSuccess) { rc = LYA_ERR_CUDA; break; }
-    if ((e = lya_alloc(&ctx->stats, ST_N + 1)) != cudaSuccess) { rc = LYA_ERR_ALLOC; break; }
+    if ((e = lya_alloc(&ctx->stats, ST_N + 1 + STEP_N)) != cudaSuccess) { rc = LYA_ERR_ALLOC; break; }
   } while (0);
   if (rc != LYA_OK) {
     lya_fail(nullptr, rc, "lya_ctx_create: %s", cudaGetErrorString(e));
@@ -261,6 +261,57 @@ extern "C" int lya_set_bins(lya_ctx* ctx, double rpmax, double rtmax, int32_t np
   ctx->bins_set = true;
   ctx->have_result = false;
   return LYA_OK;
+}
+
+// ------------------------------------------------------------------ step statistics
+// Sums over the lean forests, a warp per forest: pixels, forests, distance
+// spanned, steps, pixels of forests with a masked stretch.
+__global__ void k_steps(int64_t n, const int64_t* __restrict__ pstart, const int32_t* __restrict__ len,
+                        const uint8_t* __restrict__ flags, const double* __restrict__ dc, double* __restrict__ sums) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * blockDim.x / 32;
+  double v[STEP_N] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int64_t f = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32; f < n; f += nw) {
+    const int L = len[f];
+    if (L <= 0 || !(flags[f] & LYA_LEAN)) continue;
+    const double* d = dc + pstart[f];
+    double top = 0.0;
+    for (int k = lane; k + 1 < L; k += 32) top = fmax(top, d[k + 1] - d[k]);
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const double span = d[L - 1] - d[0];
+    v[0] += L;
+    v[1] += 1.0;
+    v[2] += span;
+    v[3] += L - 1;
+    if (top * (L - 1) > 1.5 * span) v[4] += L;
+  }
+  if (lane == 0)
+    for (int k = 0; k < STEP_N; ++k)
+      if (v[k] != 0.0) atomicAdd(&sums[k], v[k]);
+}
+
+cudaError_t lya_catalog_steps(lya_ctx* ctx, CatalogSteps* out) {
+  DevCatalog& c = ctx->cat;
+  if (!c.steps_known) {
+    double sums[STEP_N] = {};
+    double* d = reinterpret_cast<double*>(ctx->stats + ST_N + 1);
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(sums), ctx->stream);
+    if (e == cudaSuccess && c.n > 0) {
+      k_steps<<<(int)std::min<int64_t>((c.n + 3) / 4, (int64_t)ctx->num_sms * 16), 128, 0, ctx->stream>>>(
+          c.n, c.pstart, c.len, c.sorted, c.dc, d);
+      ctx->launches++;
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(sums, d, sizeof(sums), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return e;
+    c.steps.len = sums[1] > 0.0 ? sums[0] / sums[1] : 0.0;
+    c.steps.step = sums[3] > 0.0 ? sums[2] / sums[3] : 0.0;
+    c.steps.masked = sums[0] > 0.0 ? sums[4] / sums[0] : 0.0;
+    c.steps_known = true;
+  }
+  *out = c.steps;
+  return cudaSuccess;
 }
 
 // ------------------------------------------------------------------ packing
@@ -413,6 +464,7 @@ static int upload_impl(lya_ctx* ctx, int64_t n, const int64_t* start, const doub
   c.n = n; c.npix = npix; c.npad = npad; c.n_slots = n_slots;
   c.has_dl = dl != nullptr;
   c.has_moments = (omega != nullptr && odl2 != nullptr) || ingest >= 0;
+  c.steps_known = false;
   c.n_not_lean = 0;
   double *t_dc = ctx->stg.dc, *t_w = ctx->stg.w, *t_dw = ctx->stg.dw, *t_z = ctx->stg.z;
   double* t_dl = dl ? ctx->stg.dl : nullptr;

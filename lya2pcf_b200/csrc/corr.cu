@@ -1465,10 +1465,21 @@ static bool fp32_lean_walk(int variant) { return variant == 0 || variant == 3; }
 // Whether a binning is taken does then not depend on the catalogue: the walks
 // share the limit of 2,773 bins, up to which the edge tables fit for np + nt up
 // to 280 (2,500 bins: up to 380).
-static bool fp64_exact_walk(const CorrParams& p, int nb) {
+// Where it does not pay, the one-diagonal walk serves every pair:
+// * short forests, whose pairs cost the np + nt edges (and a lane its starts)
+//   whatever their length; times of the exact and of the one-diagonal walk: 8
+//   pixels, 50 x 50 bins 3.59 / 3.45 ms, 12 pixels 3.24 / 3.81 ms; 200 x 12 bins,
+//   12 pixels 4.17 / 3.85 ms, 16 pixels 3.55 / 3.67 ms; 12 x 200 bins, 18 pixels
+//   3.79 / 3.70 ms, 25 pixels 3.01 / 3.27 ms;
+// * forests with masked stretches in rp bins of less than a step: the walk passes
+//   every edge of a stretch one by one, while the other lanes wait.  1,000 forests
+//   of 325 pixels with three masked stretches: 100 x 20 bins 69 / 75 ms, 200 x 12
+//   102 / 83 ms, 600 x 3 214 / 88 ms (without the stretches 66 / 86 ms).
+static bool fp64_exact_walk(const CorrParams& p, int nb, const CatalogSteps& st) {
   constexpr size_t ROOM = 226 * 1024;
   return p.variant == 0 && corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, nb) <= ROOM &&
-         corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, nb) <= ROOM;
+         corr_smem_bytes<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, nb) <= ROOM &&
+         st.len >= std::max(13.0, (p.np + 2 * p.nt) / 18.0) && (st.masked < 0.5 || st.step * p.binner_rp <= 1.75);
 }
 
 // ------------------------------------------------------------------ CTA ranges
@@ -1532,7 +1543,8 @@ struct RunGraphKey {
   CorrParams p;
   int kind, nctas, nslots, nb;
   int slot_begin, slot_end;
-  int rest_pass;          // FP32 lean walk: second instance for the pairs it skips
+  int exact;              // FP64: the exact walk
+  int rest_pass;          // second instance, for the pairs that the lean or the exact walk skips
   int64_t n_items;
   const void* cost;
   const void* scan_tmp;
@@ -1571,7 +1583,7 @@ static cudaError_t enqueue_run(lya_ctx* ctx, const RunGraphKey& k, double* d_ran
       if (e == cudaSuccess && k.rest_pass) e = launch_corr<LYA_KERNEL_FP32_GUARDED, 16, WALK_REST>(p, k.nctas, k.nb, s);
     } else if (k.kind == LYA_KERNEL_FP32_GUARDED) {
       e = launch_corr<LYA_KERNEL_FP32_GUARDED, 16, WALK_ANY>(p, k.nctas, k.nb, s);
-    } else if (k.kind == LYA_KERNEL_FP64_DIAGONAL && fp64_exact_walk(p, k.nb)) {
+    } else if (k.kind == LYA_KERNEL_FP64_DIAGONAL && k.exact) {
       e = launch_corr<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_LEAN>(p, k.nctas, k.nb, s);
       if (e == cudaSuccess && k.rest_pass) e = launch_corr<LYA_KERNEL_FP64_DIAGONAL, 16, WALK_REST>(p, k.nctas, k.nb, s);
     } else if (k.kind == LYA_KERNEL_FP64_DIAGONAL) {
@@ -1664,7 +1676,10 @@ int lya_corr_launch(lya_ctx* ctx, const lya_corr_opts* o) {
   p.hist = ctx->hist; p.counts = ctx->counts; p.stats = ctx->stats;
   key.kind = kind; key.nctas = nctas; key.nslots = nslots; key.nb = nb; key.n_items = n;
   key.slot_begin = o->slot_begin; key.slot_end = o->slot_end;
-  const bool exact = kind == LYA_KERNEL_FP64_DIAGONAL && fp64_exact_walk(p, nb);
+  CatalogSteps steps;
+  if (kind == LYA_KERNEL_FP64_DIAGONAL && p.variant == 0) LYA_CHECK_CUDA(ctx, lya_catalog_steps(ctx, &steps));
+  const bool exact = kind == LYA_KERNEL_FP64_DIAGONAL && fp64_exact_walk(p, nb, steps);
+  key.exact = exact ? 1 : 0;
   const bool skips = exact || (kind == LYA_KERNEL_FP32_GUARDED && fp32_lean_walk(o->variant));
   key.rest_pass = skips && ctx->cat.n_not_lean > 0 ? 1 : 0;
   key.cost = ctx->cost; key.scan_tmp = ctx->scan_tmp; key.scan_bytes = scan_bytes;

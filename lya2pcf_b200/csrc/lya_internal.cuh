@@ -27,11 +27,20 @@
 
 // Device-side statistics slots (unsigned long long counters).
 enum { ST_EVALUATED = 0, ST_RECHECK = 1, ST_RUNS = 2, ST_INRANGE = 3, ST_ERROR = 4, ST_N = 8 };
+constexpr int STEP_N = 5;   // sums of k_steps
 
 // Forest catalogue on the device.  Per-pixel arrays use a padded CSR: forest f
 // owns pixels pstart[f] .. pstart[f]+len[f]-1, with pstart[f] a multiple of 4 so
 // every forest starts on a 32-byte boundary of the FP64 arrays, and
 // LYA_MARGIN zero pixels before the first and after the last forest.
+// Lengths and pixel steps of a catalogue's lean forests, by which the FP64 kernels
+// choose their walk (lya_catalog_steps).
+struct CatalogSteps {
+  double len = 0.0;      // mean number of pixels
+  double step = 0.0;     // mean distance between neighbouring pixels, Mpc/h
+  double masked = 0.0;   // share of the pixels in forests with a step above 1.5 times their mean
+};
+
 struct DevCatalog {
   int64_t n = 0;          // forests
   int64_t npix = 0;       // real pixels
@@ -63,6 +72,8 @@ struct DevCatalog {
   bool has_dl = false;
   bool has_moments = false;
   int64_t n_not_lean = 0;      // forests without the LYA_LEAN flag
+  CatalogSteps steps;          // valid with steps_known: taken when a kernel first asks after an upload
+  bool steps_known = false;
   int64_t cap_n = 0;           // allocated forests of the per-forest arrays
   int64_t cap_npad = 0;        // allocated padded pixel slots of the per-pixel arrays
 };
@@ -195,7 +206,7 @@ struct lya_ctx {
   double* get_tmp = nullptr;             // lya_corr_get's combined (hi + lo) sums, kept between calls
   int64_t get_tmp_cap = 0;
 
-  unsigned long long* stats = nullptr;   // [ST_N + 1]: counters, then the range's pair count (as double bits)
+  unsigned long long* stats = nullptr;   // [ST_N + 1 + STEP_N]: counters, the range's pair count, step sums (as double bits)
   int64_t* cta_begin = nullptr;          // [max ctas + 1]
   int32_t cta_cap = 0;
 
@@ -246,6 +257,10 @@ inline cudaError_t lya_alloc(T** p, size_t count) {
   if (lya_alloc_fault()) return cudaErrorMemoryAllocation;
   return cudaMalloc((void**)p, count * sizeof(T));
 }
+
+// The step statistics of the uploaded catalogue: one kernel and one small copy at
+// the first call after an upload.
+cudaError_t lya_catalog_steps(lya_ctx* ctx, CatalogSteps* out);
 
 // Back the pages of a host buffer that a device copy is about to fill, with
 // several threads, keeping its contents.  A copy into pages that were never

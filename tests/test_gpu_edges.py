@@ -157,3 +157,47 @@ def test_distortion_sorted_forests_of_the_general_builder(np_, nt, where):
     Do, Wo = O.distortion(fs, f1, f2, np_=np_, nt=nt)
     np.testing.assert_allclose(W, Wo, rtol=1e-12, atol=1e-12 * np.abs(Wo).max())
     assert np.abs(D - Do).max() <= 1e-10 * np.abs(Do).max() and np.abs(Do).max() > 0
+
+
+def lines(lengths, masked, seed=8):
+    """A forest of every length, within a quarter degree, steps of 2 Mpc/h; with
+    `masked`, each lacks a stretch of pixels in its middle."""
+    rng = np.random.default_rng(seed)
+    forests = []
+    for L in lengths:
+        dc = 3700.0 + 2.0 * np.arange(L) + rng.uniform(0, 60.0)
+        if masked:
+            dc[L // 2:] += 31.0
+        forests.append(dict(ra=0.5 + rng.uniform(0, 4e-3), dec=0.1 + rng.uniform(0, 4e-3), dc=dc,
+                            w=rng.uniform(0.5, 2.0, L), dw=rng.normal(0, 0.3, L), z=2.0 + 1e-3 * np.arange(L)))
+    # and one that is not sorted: the walks of sorted forests leave its pairs to a second kernel
+    forests.append(dict(forests[0], dc=np.array([3702.0, 3700.0]), w=np.ones(2), dw=np.ones(2), z=np.full(2, 2.0)))
+    return forestset(forests, pix=np.arange(len(forests)) // 8)
+
+
+@pytest.mark.parametrize('lengths,np_,nt,masked,exact', [
+    ((13,) * 12, 50, 50, False, True), ((13,) * 11 + (12,), 50, 50, False, False),
+    ((22, 23) * 6, 12, 200, False, False), ((23,) * 12, 12, 200, False, True),
+    ((120,) * 12, 200, 12, False, True), ((120,) * 12, 200, 12, True, False), ((120,) * 12, 100, 20, True, True),
+    ((120, 3) * 6, 400, 4, True, False), ((614, 1) * 3, 50, 50, True, True)])
+def test_fp64_walk_chosen(lengths, np_, nt, masked, exact):
+    """Short forests, and masked ones in narrow rp bins, take the one-diagonal
+    walk, which serves the unsorted forest in the same launch; counts and sums of
+    either as in test_fp64_walk_edges."""
+    fs = lines(lengths, masked)
+    f1, f2 = all_pairs(fs)
+    slot_start = np.searchsorted(fs.pix[f1], np.arange(fs.pix[-1] + 2))
+    hist, cnt = O.corr(fs, f1, f2, slot_start, np_=np_, nt=nt)
+    launches = {}
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        for variant in (1, 0):
+            for _ in range(2):
+                before = eng.stats()['launches']
+                launches[variant] = eng.run(kernel=N.KERNEL_FP64_DIAGONAL, variant=variant)['launches'] - before
+            h, c = eng.histograms()
+            np.testing.assert_array_equal(c, cnt)
+            for q in (N.Q_W, N.Q_RP, N.Q_RT, N.Q_Z):
+                np.testing.assert_allclose(h[:, q], hist[:, q], rtol=1e-12, atol=0)
+    assert launches[0] - launches[1] == (1 if exact else 0)
