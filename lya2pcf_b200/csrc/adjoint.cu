@@ -460,6 +460,33 @@ __global__ void k_unpad(int64_t n, const int64_t* __restrict__ start, const int6
 
 }  // namespace
 
+// Whether the band kernel takes the lean pairs.  Its table has to leave shared
+// memory for 8 warps or more (50 x 50 bins: 81 KB, 24 warps of 4.8 KB); and it has
+// to pay, by the catalogue's mean length and pixel step.  Times of the band and
+// of the gather kernel:
+// * a pair costs the band its np + nt edges and full passes of 64 rows whatever its
+//   length: 32 pixels, 50 x 50 bins 1.45 / 1.38 ms, 36 pixels 1.34 / 1.43; 200 x 12
+//   bins, 100 pixels 3.16 / 2.99, 150 pixels 5.67 / 6.24; 10 x 300 bins, 80 pixels
+//   1.76 / 1.61, 150 pixels 4.39 / 4.74; above 3,584 bins only three CTAs of the
+//   gather kernel fit an SM, and the band pays sooner: 64 x 64 bins, 20 pixels
+//   2.29 / 2.38, 32 pixels 1.70 / 2.32;
+// * a row passes its rp edges one by one: 1,000 forests of 375 pixels, 200 x 12
+//   bins (two edges a step) 32.7 / 38.1 ms, 250 x 10 38.9 / 33.3, 600 x 4 80 / 37;
+//   and rt bins in narrower rows than its four known steps: 8 x 500 44.7 / 46.6,
+//   4 x 600 35.3 / 33.2;
+// * with masked stretches (three per forest) the rows' edges have to be met in
+//   loops, and the other lanes wait: 45 x 45 bins 25.6 / 26.0 ms, 55 x 55 27.3 /
+//   26.4, 100 x 25 30.4 / 26.1, 10 x 300 28.6 / 26.4; above 3,584 bins 64 x 64
+//   33.8 / 39.8, 100 x 40 37.5 / 47.5, 200 x 20 63 / 46.
+static bool band_takes_lean(int np, int nt, int warps, double binner_rp, const CatalogSteps& st) {
+  if (warps < 8) return false;
+  const bool many = np * nt > 3584;   // gather: three CTAs per SM
+  if (st.len < (many ? 20.0 : 36.0) + 0.7 * std::max(0, np - 90) + 0.65 * std::max(0, nt - 190)) return false;
+  const double edges = st.step * binner_rp;   // rp edges a step
+  if (st.masked < 0.5) return edges <= 2.1 && nt <= 500;
+  return edges <= (many ? 1.7 : 0.5) && nt <= 200;
+}
+
 // Scratch of the adjoint, kept in the context between calls (grown, never shrunk).
 static cudaError_t adjoint_reserve(lya_ctx* ctx, int nb, int64_t n, int64_t npad, int64_t npix) {
   AdjScratch& S = ctx->adj;
@@ -488,6 +515,9 @@ int lya_adjoint_launch(lya_ctx* ctx, const double* g, double* grad_dw, double* g
   cudaStream_t s = ctx->stream;
   cudaError_t e = adjoint_reserve(ctx, nb, n, npad, npix);
   if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_ALLOC, "lya_corr_adjoint: allocation failed");
+  CatalogSteps steps;
+  e = lya_catalog_steps(ctx, &steps);
+  if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_corr_adjoint: %s", cudaGetErrorString(e));
   AdjScratch& S = ctx->adj;
   double *d_g = S.g, *coef = S.coef, *gdw = S.gdw, *gw = S.gw, *out = S.out;
   int64_t* d_start = S.start;
@@ -507,14 +537,12 @@ int lya_adjoint_launch(lya_ctx* ctx, const double* g, double* grad_dw, double* g
     p.binner_rp = (double)ctx->np / ctx->rpmax; p.binner_rt = (double)ctx->nt / ctx->rtmax;
     p.np = ctx->np; p.nt = ctx->nt; p.nb = nb; p.cos_variant = ctx->cos_variant;
     p.coef = coef; p.g_dw = gdw; p.g_w = gw;
-    // The band kernel takes the lean pairs when its table leaves shared memory
-    // for 8 warps or more (50 x 50 bins: 81 KB, 24 warps of 4.8 KB); the gather
-    // kernel takes the pairs it leaves.
+    // the band kernel, and the gather kernel for the pairs it leaves
     const size_t smem = sizeof(double) * 2 * nb, smem_max = 226 * 1024;
     const size_t table = sizeof(double) * (size_t)band_table(ctx->np, ctx->nt);
     const size_t per_warp = sizeof(double) * (size_t)band_per_warp(ctx->np, ctx->nt);
     const int warps = table < smem_max ? (int)std::min<size_t>(BAND_WARPS, (smem_max - table) / per_warp) : 0;
-    const bool band = warps >= 8;
+    const bool band = band_takes_lean(ctx->np, ctx->nt, warps, p.binner_rp, steps);
     p.skip_lean = band ? 1 : 0;
     if (band && p.n_items > 0) {
       const size_t smem_band = table + warps * per_warp;

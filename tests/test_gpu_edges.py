@@ -201,3 +201,33 @@ def test_fp64_walk_chosen(lengths, np_, nt, masked, exact):
             for q in (N.Q_W, N.Q_RP, N.Q_RT, N.Q_Z):
                 np.testing.assert_allclose(h[:, q], hist[:, q], rtol=1e-12, atol=0)
     assert launches[0] - launches[1] == (1 if exact else 0)
+
+
+@pytest.mark.parametrize('lengths,np_,nt,masked,band', [
+    ((36,) * 12, 50, 50, False, True), ((36,) * 11 + (35,), 50, 50, False, False),
+    ((112,) * 12, 200, 12, False, False), ((114,) * 12, 200, 12, False, True), ((300,) * 6, 250, 10, False, False),
+    ((130,) * 8, 10, 300, False, True), ((130,) * 8, 10, 300, True, False), ((614, 1) * 3, 4, 600, False, False),
+    ((120,) * 12, 50, 50, True, False), ((120,) * 12, 40, 40, True, True), ((120,) * 12, 64, 64, True, True),
+    ((120,) * 12, 200, 20, True, False), ((20,) * 12, 64, 64, False, True), ((20,) * 11 + (19,), 64, 64, False, False)])
+def test_adjoint_kernel_chosen(lengths, np_, nt, masked, band):
+    """Short forests, narrow rp bins and masked forests take the gather kernel,
+    which serves the unsorted forest in the same launch; gradients of either as
+    in test_adjoint_edges."""
+    fs = lines(lengths, masked)
+    f1, f2 = all_pairs(fs)
+    with PairEngine(np_=np_, nt=nt) as eng:
+        eng.upload(fs)
+        eng.set_pairs(f1, f2)
+        eng.run(kernel=N.KERNEL_FP64_PLAIN)
+        W, DW = eng.totals()
+        g = np.random.default_rng(7).normal(size=eng.nb)
+        for _ in range(2):
+            before = eng.stats()['launches']
+            gdw, gw = eng.adjoint(g)
+            launches = eng.stats()['launches'] - before
+    cdw = np.divide(g, W, out=np.zeros_like(W), where=W != 0)
+    odw, ow = O.adjoint(fs, f1, f2, cdw, -cdw * np.divide(DW, W, out=np.zeros_like(W), where=W != 0), np_=np_, nt=nt)
+    assert np.abs(odw).max() > 0
+    np.testing.assert_allclose(gdw, odw, rtol=0, atol=1e-11 * np.abs(odw).max())
+    np.testing.assert_allclose(gw, ow, rtol=0, atol=1e-11 * np.abs(ow).max())
+    assert launches == (5 if band else 4)   # coefficients, pair kernels, two copies
