@@ -168,6 +168,9 @@ __global__ void k_count_zero_diag(int nb, const double* __restrict__ cov, unsign
     if (cov[(size_t)b * nb + b] == 0.0) atomicAdd(zero, 1ull);
 }
 
+// Row data beyond this is given back after the call (676 rows of 2,500 bins take 41 MB).
+constexpr int64_t KEEP_ROWS = (int64_t(256) << 20) / sizeof(double);
+
 // Room for `rows` doubles of row data, nb bins and `mat` matrix entries.
 cudaError_t cov_reserve(CovScratch& c, int64_t rows, int nb, int64_t mat) {
   cudaError_t e = cudaSuccess;
@@ -241,6 +244,10 @@ extern "C" int lya_covariance(lya_ctx* ctx, int64_t n_rows, const double* xi, co
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   float ms = 0.f;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+  if (ctx->covs.cap_rows > KEEP_ROWS) {
+    lya_free(ctx->covs.rows);
+    ctx->covs.cap_rows = 0;
+  }
   if (e != cudaSuccess) return lya_fail(ctx, LYA_ERR_CUDA, "lya_covariance: %s", cudaGetErrorString(e));
   ctx->last.kernel_ms = ms;
   if (nzero) return lya_fail(ctx, LYA_ERR_DATA, "lya_covariance: %llu bins have zero total weight", nzero);

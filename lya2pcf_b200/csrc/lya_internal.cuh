@@ -228,8 +228,8 @@ struct lya_ctx {
   int32_t dist_shape = 0;                // lya_dist_config: launch shape of the distortion kernel
   int64_t dist_max_items = 0;            // lya_dist_config: 0 = every forest pair, else the first n
 
-  // covariance post-processing: scratch kept between calls (grown, never
-  // shrunk), and the last covariance, kept for lya_covariance_smooth
+  // covariance post-processing: scratch kept between calls (row data up to 256
+  // MB), and the last covariance, kept for lya_covariance_smooth
   CovScratch covs;
   double* cov = nullptr;                 // [cov_nb][cov_nb]
   int32_t cov_nb = 0;

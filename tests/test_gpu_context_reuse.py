@@ -104,3 +104,29 @@ def test_device_memory_as_a_host_output_is_refused(nb_side):
         N.check(eng.lib.lya_covariance_smooth(eng.ctx, None, N.ptr(smooth), C.byref(sm)), eng.ctx)
         assert sm.value == 1 and np.isfinite(smooth).all()
     assert float(dev.abs().max()) == 0.0
+
+
+def test_covariance_gives_large_row_scratch_back():
+    """5,000 rows of 2,500 bins pass through 300 MB of device scratch, which an
+    engine that lives on does not hold; 100 rows keep theirs (6 MB)."""
+    import torch
+    rng = np.random.default_rng(4)
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    with PairEngine() as eng:
+        mean, c = np.zeros(2500), np.zeros((2500, 2500))
+
+        def cov(n):
+            xi, w = rng.normal(size=(n, 2500)), rng.uniform(1.0, 2.0, (n, 2500))
+            N.check(eng.lib.lya_covariance(eng.ctx, n, N.ptr(xi), N.ptr(w), N.ptr(mean), N.ptr(c)), eng.ctx)
+            xm = (xi * w).sum(0) / w.sum(0)
+            np.testing.assert_allclose(mean, xm, rtol=1e-12, atol=1e-14)
+            y = w * (xi - xm)
+            k = rng.integers(0, 2500, 40)
+            np.testing.assert_allclose(c[np.ix_(k, k)], (y.T[k] @ y[:, k]) / np.outer(w.sum(0), w.sum(0))[np.ix_(k, k)],
+                                       rtol=0, atol=1e-12 * np.abs(np.diag(c)).max())
+
+        cov(100)
+        before = free()
+        cov(5000)
+        assert free() >= before - (8 << 20)
+        cov(100)
