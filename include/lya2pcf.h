@@ -52,10 +52,13 @@ typedef struct {
                               coordinates -- for pairs of sorted forests with
                               0 <= dc < 1e6, walk 2 for the others; FP64: two
                               diagonals per lane and exact bin edges for the
-                              same pairs, walk 1 for the others and for
-                              binnings whose edges do not fit shared memory),
+                              same pairs, walk 1 for the others, for binnings
+                              whose edges do not fit shared memory and for
+                              catalogues of short forests, or of masked ones
+                              in narrow rp bins),
                               1 = one diagonal per lane,
-                              2 = two diagonals per lane, 3 = same as 0 */
+                              2 = two diagonals per lane, 3 = same as 0 (FP32
+                              kernel only) */
   int32_t run_cap;         /* longest register run of the diagonal walks before it
                               is recorded (bounds FP32 run sums): 0 = default
                               (128), else a power of two in [8, 1024] */

@@ -6,8 +6,8 @@ pixels and the pair bins held fixed (bins depend only on comoving distances and
 directions, which are not differentiated).
 
 * :func:`xi` -- ``torch.autograd.Function`` mapping per-pixel (w, dw) tensors to
-  xi[np*nt]; its backward calls ``lya_corr_adjoint`` (a gather over both
-  directions of every forest pair, no stored pairs).
+  xi[np*nt]; its backward calls ``lya_corr_adjoint`` (one pass over every forest
+  pair serves both its forests, or a gather in either direction; no stored pairs).
 * :func:`project_delta` -- the mean-and-slope projection of
   ``forest_class.fill_dw(project=True)`` (``forest_class.py:48-68``) in torch, so
   gradients chain from xi to the raw deltas and weights.

@@ -7,9 +7,10 @@
 // and symmetrically for j.  Bins with W_b == 0 contribute nothing (xi_b = 0,
 // as post_processing.py:147 defines it).
 //
-// Two kernels share the work queue.  k_adjoint_band takes every pair of forests
-// whose dc are sorted, finite and not negative (the LYA_LEAN flag) and serves
-// both forests of a pair in one pass; k_adjoint takes the others: the gather
+// Two kernels share the work queue.  k_adjoint_band takes the pairs of forests
+// whose dc are sorted, finite and not negative (the LYA_LEAN flag), where that
+// pays (band_takes_lean), and serves both forests of a pair in one pass;
+// k_adjoint takes the others: the gather
 // form, walked in both directions, one lane per pixel i over its partners j,
 // every bin from the reference FP64 formula.  The pair bin is symmetric under
 // the swap (|dc1-dc2|, dc1+dc2 and the FMA-ordered cos12 are).
@@ -190,8 +191,9 @@ constexpr int BAND_RING = 128;   // f2 pixels in a warp's ring: 64 in use, 32 ah
 
 // Shared memory, as offsets in doubles: the coefficients (2 values) of the nt
 // bins of every number of rp edges passed (0 .. 2 np, the first and the last out
-// of range), then per warp the ring (w, dw) of even and odd pixels, the ring's distances, the (grad dw, grad w) of 32 finished f2
-// pixels, the rp edges [2 np + 1] and the rt edges [nt + 1].
+// of range), then per warp the ring (w, dw) of even and odd pixels, the ring's
+// distances, the (grad dw, grad w) of 32 finished f2 pixels, the rp edges
+// [2 np + 1] and the rt edges [nt + 1].
 constexpr int BAND_D = 2 * BAND_RING, BAND_OUT = BAND_D + BAND_RING, BAND_EX = BAND_OUT + 64;
 __host__ __device__ __forceinline__ int band_table(int np, int nt) { return 2 * (2 * np + 1) * nt; }
 __host__ __device__ __forceinline__ int band_per_warp(int np, int nt) { return BAND_EX + ((2 * np + 1 + nt + 1 + 1) & ~1); }
@@ -200,10 +202,10 @@ extern __shared__ __align__(16) double s_band[];
 __device__ __forceinline__ double band_d(int at) { return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(s_band) + at); }
 __device__ __forceinline__ double2 band_d2(int at) { return *reinterpret_cast<const double2*>(reinterpret_cast<const char*>(s_band) + at); }
 
-// Bin state of a row: the byte offsets ox of the next rp edge and oc of
-// the bin's coefficients, the next rp edge, and the steps of its next four rt
-// edges (kt, then kt2: 16 bits each, the nearest lowest).  The row's partners are in range on
-// steps kb .. kb + kn - 1.
+// Bin state of a row: the byte offsets ox of the next rp edge and oc of the bin's
+// coefficients, the next rp edge, and the steps of its next four rt edges (kt,
+// then kt2: 16 bits each, the nearest lowest).  The row's partners are in range
+// on steps kb .. kb + kn - 1.
 struct BandRow {
   double d, w, dw;
   double ex;

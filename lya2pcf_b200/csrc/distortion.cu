@@ -22,16 +22,17 @@
 // column of a pixel spans a few rt bins only, so the column products are
 // 50x50 dense blocks (rp x rp) per pair of rt bins.
 //
-// One CTA per forest pair (dynamic queue).  Bins come from the reference FP64
-// formula.  Phase 1: the columns of every pixel (a warp per pixel, lanes over
-// its partners) go to CTA-private global scratch as dense [TS rt bins][np]
-// rows.  Phase 2: the 50x50 (rp x rp) blocks (t, u) of D over the pair's window
-// of rt bins, diagonal blocks first (they complete the moments of bin t, read
-// from the same staged rows: the f1 weights placed in padding columns
-// NS..NS+3 of the staged rows make accumulator columns NS..NS+3 of the diagonal
-// block's MMAs the four moments, when NS + 4 <= 64; otherwise a loop over the
-// staged rows; a diagonal block is symmetric, so only the tiles that reach its
-// upper triangle are multiplied).  A block whose rt bins are both spanned by some
+// One CTA per forest pair (dynamic queue).  Bins are those of the reference FP64
+// formula.  Phase 1: the columns of every pixel go to CTA-private global scratch
+// as dense [TS rt bins][np] rows, from exact bin edges for pairs of long lean
+// forests (build_columns, lanes over the bins), otherwise from the bin of every
+// pixel pair (a warp per pixel, lanes over its partners).  Phase 2: the 50x50
+// (rp x rp) blocks (t, u) of D over the pair's window of rt bins, diagonal blocks
+// first (they complete the moments of bin t, read from the same staged rows: the
+// f1 weights placed in padding columns NS..NS+3 of the staged rows make
+// accumulator columns NS..NS+3 of the diagonal block's MMAs the four moments, when
+// NS + 4 <= 64; otherwise a loop over the staged rows; a diagonal block is
+// symmetric, so only the tiles that reach its upper triangle are multiplied).  A block whose rt bins are both spanned by some
 // pixel column gets the column products as a small dense FP64 GEMM on the
 // tensor cores: the rows of the pixels covering t and u are staged in shared
 // memory in chunks of CH pixels, and each warp accumulates 16 x 8 tiles of the
@@ -600,10 +601,10 @@ __global__ void __launch_bounds__(DT, 1) k_dist(const DistParams p) {
     // ms (72,415 forest pairs) against a list, an exposed first chunk and two
     // barriers a chunk for each block.  Blocks with d >= maxspan have no column
     // products and come last, without barriers.
-    // Bound: the FP64 MMAs of the blocks (about 35 of the 137 ms at their peak
-    // rate) and the column build, which follow each other in a CTA, issue 46% busy
-    // on the whole; two CTAs of 256 threads per SM, which would overlap them,
-    // take 157.8 ms (chunks of 16, shared loads per MMA).
+    // Bound: the FP64 MMAs of the blocks (27 of the 137 ms at their peak rate) and
+    // the column build, which follow each other in a CTA, issue 46% busy on the
+    // whole; two CTAs of 256 threads per SM, which would overlap them, take 157.8
+    // ms (chunks of 16, shared loads per MMA).
     const int SET = CH * NPAD;   // doubles of one row set
     // pixels whose column spans both t and u = t + d, into list l
     auto build_list = [&](int t, int d, int l, int* cnt) {

@@ -178,9 +178,10 @@ class PairEngine:
         catalogue: time every candidate on a contiguous range of owner slots
         holding about ``fraction`` of the work queue's pixel pairs (the second
         of two runs, so each candidate is timed from its captured graph) and
-        keep the fastest for later :meth:`run` calls.  Walks: 0 (the FP32
-        kernel's lean walk, two diagonals per lane otherwise), 2 (two
-        diagonals per lane) and 1 (one per lane).  Returns the timings."""
+        keep the fastest for later :meth:`run` calls.  Walks: 0 (the kernel's
+        default: the lean walk of the FP32 kernel, the exact walk of the FP64
+        kernel where it pays), 2 (two diagonals per lane) and 1 (one per lane,
+        FP32 kernel).  Returns the timings."""
         if variants is None:
             variants = (0, 2, 1) if int(kernel) == N.KERNEL_FP32_GUARDED else (0, 2)
         slots = self._sample_slots(fraction, seed)
