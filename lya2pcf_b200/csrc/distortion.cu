@@ -32,15 +32,15 @@
 // f1 weights placed in padding columns NS..NS+3 of the staged rows make
 // accumulator columns NS..NS+3 of the diagonal block's MMAs the four moments, when
 // NS + 4 <= 64; otherwise a loop over the staged rows; a diagonal block is
-// symmetric, so only the tiles that reach its upper triangle are multiplied).  A block whose rt bins are both spanned by some
-// pixel column gets the column products as a small dense FP64 GEMM on the
-// tensor cores: the rows of the pixels covering t and u are staged in shared
-// memory in chunks of CH pixels, and each warp accumulates 16 x 8 tiles of the
-// block (four tiles of 16 rp bins down, 8 across; mma.sync m16n8k8 f64, FP64
-// having no tcgen05 kind; rows at or beyond np enter as zeros); the
-// rank-4 and diagonal terms are added to the accumulators, and each D entry of
-// the window gets one atomic add per forest pair (both (A, B) and (B, A): D is
-// symmetric).
+// symmetric, so only the tiles that reach its upper triangle are multiplied).  A
+// block whose rt bins are both spanned by some pixel column gets the column
+// products as a small dense FP64 GEMM on the tensor cores: the rows of the pixels
+// covering t and u are staged in shared memory in chunks of CH pixels, and each
+// warp accumulates 16 x 8 tiles of the block (four tiles of 16 rp bins down, 8
+// across; mma.sync m16n8k8 f64, FP64 having no tcgen05 kind; rows at or beyond np
+// enter as zeros); the rank-4 and diagonal terms are added to the accumulators,
+// and each D entry of the window gets one atomic add per forest pair (both (A, B)
+// and (B, A): D is symmetric).
 // A forest whose sum w dl^2 is 0 has no slope to project out: its slope terms
 // are 0.
 #include <cuda_pipeline.h>
